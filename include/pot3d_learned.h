@@ -19,11 +19,24 @@ extern "C" {
  * 0; *err (device int) is set if a bounded wait ran out. */
 int pot3d_tc_gemm(const void *A, const void *B, void *D, const float *bias, int batch, int M, int N, int K,
                   long long ldd, long long bstride_d, int accumulate, int out_bf16, int *err, void *stream);
+/* The same with a GELU of the result (act, not with accumulate), and with K
+ * split over `splits` blocks per output tile (FP32 output; ws: splits * batch
+ * * M * N floats), for products with few tiles and a long K. */
+int pot3d_tc_gemm_ex(const void *A, const void *B, void *D, const float *bias, int batch, int M, int N, int K,
+                     long long ldd, long long bstride_d, int accumulate, int out_bf16, int act, int splits, float *ws,
+                     int *err, void *stream);
 
 /* 4-D permutation out[o] = in[i], i[perm[a]] = o[a], zero outside in
  * (padding/cropping); dtypes 0 = FP32, 1 = BF16; add: FP32 out += value. */
 int pot3d_fno_permute(const void *in, int in_dt, const long long *in_dims, void *out, int out_dt,
                       const long long *out_dims, const int *perm, int add, void *stream);
+
+/* A Fourier layer's sum and activation: pre[m][c] + spec[b][c][ph][th] (spec
+ * BF16 [B][W][nph][Pth], m = (b, ph, th), pre FP32 [B*nph*nth][W]; stored back
+ * into pre with keep != 0), its GELU with act != 0, into vout BF16 [m][64],
+ * zero past W <= 64. */
+int pot3d_fno_spec_act(float *pre, const void *spec, int B, int W, int nph, int nth, int Pth, int act, int keep,
+                       void *vout, void *stream);
 
 /* GELU (tanh form) of pre[M][C] into out (zero-padded to ldo columns), or
  * with backward != 0 the incoming gradient times GELU'(pre). */
@@ -38,6 +51,11 @@ int pot3d_fno_colsum(const float *in, long long M, int C, int ld, float *out, in
  * gradient scaled by `scale`. */
 int pot3d_fno_relmse(const float *pred, int ldp, const void *tgt, int t_dt, int nbatch, long long npos, int R,
                      float scale, float *grad, float *loss, void *stream);
+/* The same with the caller's scratch (device floats, pot3d_fno_relmse_scratch
+ * of them) instead of a stream-ordered allocation. */
+int pot3d_fno_relmse_scratch(int nbatch);
+int pot3d_fno_relmse_ws(const float *pred, int ldp, const void *tgt, int t_dt, int nbatch, long long npos, int R,
+                        float scale, float *grad, float *loss, float *ws, void *stream);
 
 /* One Adam step on FP32 weights w with gradient g (moments m1, m2); writes
  * a BF16 copy into wb when wb is not NULL. */

@@ -10,7 +10,10 @@
 //   pot3d_fno_adam     Adam step on FP32 master weights with a BF16 copy
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <stdint.h>
 
+#include "../../include/pot3d_learned.h"
+#include "fno_math.cuh"
 #include "pot3d_internal.cuh"
 
 namespace {
@@ -34,80 +37,154 @@ struct Dims4 {
 
 // out[o0][o1][o2][o3] = in[i] with i[perm[a]] = o[a]; zero where i is
 // outside in's extent.  With add, out (FP32) += value.
-__global__ void k_permute(const void *__restrict__ in, int in_dt, Dims4 id, void *__restrict__ out, int out_dt, Dims4 od,
-                          int p0, int p1, int p2, int p3, int add) {
-  const long long n = od.d[0] * od.d[1] * od.d[2] * od.d[3];
-  const int perm[4] = {p0, p1, p2, p3};
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    long long o[4];
-    long long r = t;
-    o[3] = r % od.d[3];
-    r /= od.d[3];
-    o[2] = r % od.d[2];
-    r /= od.d[2];
-    o[1] = r % od.d[1];
-    o[0] = r / od.d[1];
-    long long i[4];
-    bool inside = true;
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-      i[perm[a]] = o[a];
-    }
-#pragma unroll
-    for (int a = 0; a < 4; a++) inside = inside && i[a] < id.d[a];
-    float v = 0.0f;
-    if (inside) v = ld(in, ((i[0] * id.d[1] + i[1]) * id.d[2] + i[2]) * id.d[3] + i[3], in_dt);
-    if (add)
-      reinterpret_cast<float *>(out)[t] += v;
-    else
-      st(out, t, out_dt, v);
+struct PermArgs {
+  const void *in;
+  void *out;
+  int in_dt, out_dt, add;
+  long long is[4];  // in's stride along each out axis
+  long long ie[4];  // in's extent along each out axis
+  long long od[4];
+};
+__device__ __forceinline__ void perm_put(const PermArgs &a, long long t, float v) {
+  if (a.add)
+    reinterpret_cast<float *>(a.out)[t] += v;
+  else
+    st(a.out, t, a.out_dt, v);
+}
+// in's fastest axis is out's: whole rows, a warp a row (one set of divisions
+// per row instead of per element).
+__global__ void __launch_bounds__(256) k_permute_rows(PermArgs a, long long rows) {
+  const int lane = threadIdx.x & 31;
+  for (long long r = blockIdx.x * 8LL + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8LL) {
+    const long long o01 = r / a.od[2];
+    const long long o2 = r % a.od[2], o1 = o01 % a.od[1], o0 = o01 / a.od[1];
+    const bool inside = o0 < a.ie[0] && o1 < a.ie[1] && o2 < a.ie[2];
+    const long long ib = o0 * a.is[0] + o1 * a.is[1] + o2 * a.is[2];
+    for (long long c = lane; c < a.od[3]; c += 32)
+      perm_put(a, r * a.od[3] + c, inside && c < a.ie[3] ? ld(a.in, ib + c, a.in_dt) : 0.0f);
   }
 }
-
-__device__ __forceinline__ float gelu_f(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  return 0.5f * x * (1.0f + tanhf(k0 * (x + k1 * x * x * x)));
+// in's fastest axis is out axis q < 3: tiles of PT3 x 32 over (3, q) turned
+// in shared memory, so both sides move whole lines.  u, v: the other two out
+// axes.
+constexpr int PT3 = 128;
+struct TileArgs {
+  const void *in;
+  void *out;
+  long long is3, isu, isv, osq, osu, osv;  // strides along out axes 3, u, v (in) and q, u, v (out)
+  long long ieq, ie3, ieu, iev, odq, od3;  // extents (in's along out axes)
+  unsigned n3, nq, nv;                     // tiles along 3 and q; out's extent along v
+  int add;
+};
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(256) k_permute_tile(const __grid_constant__ TileArgs a) {
+  __shared__ float tile[PT3][33];
+  const unsigned bl = blockIdx.x;  // below 2^31
+  const unsigned i3 = bl % a.n3, iq = bl / a.n3 % a.nq, uv = bl / a.n3 / a.nq;
+  const long long b3 = (long long)i3 * PT3, bq = (long long)iq * 32;
+  const long long ov = uv % a.nv, ou = uv / a.nv;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const bool inside = ou < a.ieu && ov < a.iev && bq + x < a.ieq;
+  const TI *ib = reinterpret_cast<const TI *>(a.in) + ou * a.isu + ov * a.isv + bq + x;
+  TI r[PT3 / 8];
+#pragma unroll
+  for (int k = 0; k < PT3 / 8; k++) {
+    const long long o3 = b3 + y + 8 * k;
+    r[k] = inside && o3 < a.ie3 ? ib[o3 * a.is3] : TI(0.0f);
+  }
+#pragma unroll
+  for (int k = 0; k < PT3 / 8; k++) tile[y + 8 * k][x] = (float)r[k];
+  __syncthreads();
+  const long long ob = ou * a.osu + ov * a.osv + b3 + x;
+  TO *out = reinterpret_cast<TO *>(a.out);
+#pragma unroll
+  for (int s = 0; s < 4; s++) {
+    const long long oq = bq + y + 8 * s;
+    if (oq >= a.odq) break;
+#pragma unroll
+    for (int k = 0; k < PT3 / 32; k++) {
+      if (b3 + x + 32 * k < a.od3) {
+        TO *o = out + ob + oq * a.osq + 32 * k;
+        const float val = tile[x + 32 * k][y + 8 * s];
+        if (a.add)
+          *o = (TO)((float)*o + val);  // FP32 only
+        else
+          *o = (TO)val;
+      }
+    }
+  }
 }
-__device__ __forceinline__ float gelu_d(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  const float u = k0 * (x + k1 * x * x * x);
-  const float t = tanhf(u);
-  return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * k0 * (1.0f + 3.0f * k1 * x * x);
+// One Fourier layer's sum and activation: pre[m][c] += spec[b][c][ph][th] for
+// m = (b, ph, th), and vout[m][0..63] (BF16) = act(pre[m][c]), zero for c >= W.
+// keep: pre's sum is stored (the backward pass needs it).  The spectral term
+// is turned in shared memory (32 theta points at once).
+__global__ void __launch_bounds__(256) k_spec_act(float *__restrict__ pre, const __nv_bfloat16 *__restrict__ spec, int W,
+                                                  int nph, int nth, int Pth, int act, int keep,
+                                                  __nv_bfloat16 *__restrict__ vout) {
+  __shared__ float tile[64][33];
+  const int lane = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int tiles = (nth + 31) / 32, th0 = (int)(blockIdx.x % tiles) * 32;
+  const int line = blockIdx.x / tiles, b = line / nph, ph = line % nph;
+  for (int c = y; c < W; c += 8)
+    if (th0 + lane < nth)
+      tile[c][lane] = __bfloat162float(spec[(((long long)b * W + c) * nph + ph) * Pth + th0 + lane]);
+  __syncthreads();
+#pragma unroll
+  for (int r = y; r < 32; r += 8) {
+    const int th = th0 + r;
+    if (th >= nth) break;
+    const long long m = (long long)line * nth + th;
+#pragma unroll
+    for (int c = lane; c < 64; c += 32) {
+      float v = 0.0f;
+      if (c < W) {
+        v = pre[m * W + c] + tile[c][r];
+        if (keep) pre[m * W + c] = v;
+        if (act) v = gelu_f(v);
+      }
+      vout[m * 64 + c] = __float2bfloat16_rn(v);
+    }
+  }
 }
 
 // forward: out[m][c] = gelu(pre[m][c]) for c < C, 0 for C <= c < ldo.
 // backward: out[m][c] = grad[m][c] * gelu'(pre[m][c]) (c < C), 0 beyond.
-__global__ void k_gelu(const float *__restrict__ pre, long long M, int C, int ldp, const void *__restrict__ grad,
-                       int g_dt, int ldg, void *__restrict__ out, int out_dt, int ldo, int backward) {
-  const long long n = M * ldo;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long m = t / ldo;
-    const int c = (int)(t % ldo);
-    float v = 0.0f;
-    if (c < C) {
-      const float x = pre[m * ldp + c];
-      v = backward ? ld(grad, m * ldg + c, g_dt) * gelu_d(x) : gelu_f(x);
+__global__ void __launch_bounds__(256) k_gelu(const float *__restrict__ pre, long long M, int C, int ldp,
+                                              const void *__restrict__ grad, int g_dt, int ldg, void *__restrict__ out,
+                                              int out_dt, int ldo, int backward) {
+  const int lane = threadIdx.x & 31;
+  for (long long m = blockIdx.x * 8LL + (threadIdx.x >> 5); m < M; m += gridDim.x * 8LL)
+    for (int c = lane; c < ldo; c += 32) {
+      float v = 0.0f;
+      if (c < C) {
+        const float x = pre[m * ldp + c];
+        v = backward ? ld(grad, m * ldg + c, g_dt) * gelu_d(x) : gelu_f(x);
+      }
+      st(out, m * ldo + c, out_dt, v);
     }
-    st(out, t, out_dt, v);
-  }
 }
 
-// out[c] = sum_m in[m][c], c < C: per-block partial sums in a fixed order.
-__global__ void k_colsum(const float *__restrict__ in, long long M, int C, int ld, float *__restrict__ part) {
-  const int c = blockIdx.y;
+// out[c] = sum_m in[m][c], c < C: per-block partial sums in a fixed order.  A
+// block sums 32 columns (a lane a column, so a warp reads a line of a row).
+constexpr int CS_ROWS = 32;  // rows a block reads at once
+__global__ void __launch_bounds__(32 * CS_ROWS) k_colsum(const float *__restrict__ in, long long M, int C, int ld,
+                                                         float *__restrict__ part) {
+  const int lane = threadIdx.x & 31, y = threadIdx.x >> 5, c = blockIdx.y * 32 + lane;
   float s = 0.0f;
-  for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < M; m += (long long)gridDim.x * blockDim.x)
-    s += in[m * ld + c];
-  __shared__ float red[256];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
+  if (c < C) {
+#pragma unroll 8
+    for (long long m = blockIdx.x * (long long)CS_ROWS + y; m < M; m += gridDim.x * (long long)CS_ROWS)
+      s += in[m * ld + c];
   }
-  if (threadIdx.x == 0) part[(long long)c * gridDim.x + blockIdx.x] = red[0];
+  __shared__ float red[CS_ROWS][32];
+  red[y][lane] = s;
+  __syncthreads();
+  if (y == 0 && c < C) {
+    float t = 0.0f;
+#pragma unroll
+    for (int q = 0; q < CS_ROWS; q++) t += red[q][lane];
+    part[(long long)c * gridDim.x + blockIdx.x] = t;
+  }
 }
 __global__ void k_colsum_final(const float *__restrict__ part, int nb, int C, float *__restrict__ out, int add) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -118,41 +195,80 @@ __global__ void k_colsum_final(const float *__restrict__ part, int nb, int C, fl
 }
 
 // Per sample b: loss_b = sum (pred - tgt)^2 / sum tgt^2 over npos x R values;
-// grad = 2 (pred - tgt) / sum tgt^2 * scale.  pred rows have ldp >= R.
-__global__ void k_relmse(const float *__restrict__ pred, int ldp, const void *__restrict__ tgt, int t_dt,
-                         long long npos, int R, float scale, float *__restrict__ grad, float *__restrict__ loss) {
-  const int b = blockIdx.x;
+// grad = 2 (pred - tgt) / sum tgt^2 * scale.  pred rows have ldp >= R.  Three
+// launches: RM_BLOCKS partial sums a sample, their total in a fixed order, the
+// gradient.  (One block a sample did both passes over a sample's 8 million
+// values alone: 38 ms for four 127x181x361 samples, against 0.2 ms.)
+constexpr int RM_BLOCKS = 256;
+constexpr int RM_POS = 8;  // positions a block takes at once, one per warp
+__global__ void __launch_bounds__(256) k_relmse_part(const float *__restrict__ pred, int ldp,
+                                                     const void *__restrict__ tgt, int t_dt, long long npos, int R,
+                                                     float *__restrict__ part) {
+  const int b = blockIdx.y, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const float *pb = pred + (long long)b * npos * ldp;
+  const long long tb = (long long)b * npos * R;
+  float se = 0.0f, st2 = 0.0f;
+  for (long long p = (long long)blockIdx.x * RM_POS + w; p < npos; p += (long long)RM_BLOCKS * RM_POS) {
+    for (int c = lane; c < R; c += 32) {
+      const float tv = ld(tgt, tb + p * R + c, t_dt);
+      const float d = pb[p * ldp + c] - tv;
+      se += d * d;
+      st2 += tv * tv;
+    }
+  }
+  __shared__ float r1[8], r2[8];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    se += __shfl_xor_sync(0xffffffffu, se, o);
+    st2 += __shfl_xor_sync(0xffffffffu, st2, o);
+  }
+  if (lane == 0) {
+    r1[w] = se;
+    r2[w] = st2;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float a = 0.0f, c = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      a += r1[q];
+      c += r2[q];
+    }
+    part[2 * (b * RM_BLOCKS + blockIdx.x)] = a;
+    part[2 * (b * RM_BLOCKS + blockIdx.x) + 1] = c;
+  }
+}
+// den[b] and loss[b] from the sample's partial sums (one warp a sample).
+__global__ void k_relmse_sum(const float *__restrict__ part, float *__restrict__ den, float *__restrict__ loss) {
+  const int b = blockIdx.x, lane = threadIdx.x;
+  float se = 0.0f, st2 = 0.0f;
+  for (int q = lane; q < RM_BLOCKS; q += 32) {
+    se += part[2 * (b * RM_BLOCKS + q)];
+    st2 += part[2 * (b * RM_BLOCKS + q) + 1];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    se += __shfl_xor_sync(0xffffffffu, se, o);
+    st2 += __shfl_xor_sync(0xffffffffu, st2, o);
+  }
+  if (lane == 0) {
+    const float d = fmaxf(st2, 1e-30f);
+    den[b] = d;
+    loss[b] = se / d;
+  }
+}
+__global__ void __launch_bounds__(256) k_relmse_grad(const float *__restrict__ pred, int ldp,
+                                                     const void *__restrict__ tgt, int t_dt, long long npos, int R,
+                                                     float scale, const float *__restrict__ den,
+                                                     float *__restrict__ grad) {
+  const int b = blockIdx.y, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const float *pb = pred + (long long)b * npos * ldp;
   float *gb = grad + (long long)b * npos * ldp;
   const long long tb = (long long)b * npos * R;
-  __shared__ float r1[256], r2[256];
-  float se = 0.0f, st2 = 0.0f;
-  for (long long t = threadIdx.x; t < npos * R; t += blockDim.x) {
-    const long long p = t / R;
-    const int c = (int)(t % R);
-    const float tv = ld(tgt, tb + t, t_dt);
-    const float d = pb[p * ldp + c] - tv;
-    se += d * d;
-    st2 += tv * tv;
-  }
-  r1[threadIdx.x] = se;
-  r2[threadIdx.x] = st2;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) {
-      r1[threadIdx.x] += r1[threadIdx.x + o];
-      r2[threadIdx.x] += r2[threadIdx.x + o];
-    }
-    __syncthreads();
-  }
-  const float den = fmaxf(r2[0], 1e-30f);
-  if (threadIdx.x == 0) loss[b] = r1[0] / den;
-  const float f = 2.0f * scale / den;
-  for (long long t = threadIdx.x; t < npos * ldp; t += blockDim.x) {
-    const long long p = t / ldp;
-    const int c = (int)(t % ldp);
-    gb[t] = c < R ? f * (pb[t] - ld(tgt, tb + p * R + c, t_dt)) : 0.0f;
-  }
+  const float f = 2.0f * scale / den[b];
+  for (long long p = (long long)blockIdx.x * RM_POS + w; p < npos; p += (long long)gridDim.x * RM_POS)
+    for (int c = lane; c < ldp; c += 32)
+      gb[p * ldp + c] = c < R ? f * (pb[p * ldp + c] - ld(tgt, tb + p * R + c, t_dt)) : 0.0f;
 }
 
 __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m1, float *__restrict__ m2,
@@ -173,20 +289,28 @@ __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float
 }
 
 // x[b][p][0] = br0n[b][p]; x[b][p][1..3] = consts[p][0..2]; other channels 0.
+// Eight channels (16 bytes) per thread.
 __global__ void k_inputs(const float *__restrict__ br0n, const float *__restrict__ consts, long long B, long long npos,
-                         __nv_bfloat16 *__restrict__ x) {
-  const long long n = B * npos * 64;
+                         __nv_bfloat16 *__restrict__ x, int aligned) {
+  const long long n = B * npos * 8;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(t & 63);
-    const long long bp = t >> 6;
-    const long long p = bp % npos;
-    float v = 0.0f;
-    if (c == 0)
-      v = br0n[bp];
-    else if (c < 4)
-      v = consts[p * 3 + (c - 1)];
-    x[t] = __float2bfloat16_rn(v);
+    uint4 w = make_uint4(0u, 0u, 0u, 0u);
+    if ((t & 7) == 0) {
+      const long long bp = t >> 3, p = B == 1 ? bp : bp % npos;
+      const __nv_bfloat162 a = __float22bfloat162_rn(make_float2(br0n[bp], consts[p * 3])),
+                           b = __float22bfloat162_rn(make_float2(consts[p * 3 + 1], consts[p * 3 + 2]));
+      w.x = *reinterpret_cast<const unsigned *>(&a);
+      w.y = *reinterpret_cast<const unsigned *>(&b);
+    }
+    if (aligned) {
+      reinterpret_cast<uint4 *>(x)[t] = w;
+    } else {
+      const unsigned h[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        reinterpret_cast<unsigned short *>(x)[8 * t + q] = (unsigned short)(h[q >> 1] >> (16 * (q & 1)));
+    }
   }
 }
 
@@ -213,10 +337,55 @@ extern "C" int pot3d_fno_permute(const void *in, int in_dt, const long long *in_
     pot3d_set_error("pot3d_fno_permute: add needs an FP32 output");
     return POT3D_ERR_ARG;
   }
-  const long long n = od.d[0] * od.d[1] * od.d[2] * od.d[3];
-  k_permute<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(in, in_dt, id, out, out_dt, od, perm[0], perm[1], perm[2],
-                                                            perm[3], add);
+  PermArgs a{in, out, in_dt, out_dt, add, {}, {}, {}};
+  long long is[4] = {0, 0, 0, 1};
+  for (int x = 2; x >= 0; x--) is[x] = is[x + 1] * id.d[x + 1];
+  int q = 3;
+  for (int x = 0; x < 4; x++) {
+    a.is[x] = is[perm[x]];
+    a.ie[x] = id.d[perm[x]];
+    a.od[x] = od.d[x];
+    if (perm[x] == 3) q = x;
+  }
+  cudaStream_t s = (cudaStream_t)stream;
+  if (q == 3) {
+    const long long rows = od.d[0] * od.d[1] * od.d[2];
+    k_permute_rows<<<grid_for(rows * 32), 256, 0, s>>>(a, rows);
+  } else {
+    const int u = q == 0 ? 1 : 0, v = q == 2 ? 1 : 2;
+    const long long tq = (od.d[q] + 31) / 32, t3 = (od.d[3] + PT3 - 1) / PT3, nb = tq * t3 * od.d[u] * od.d[v];
+    if (nb > 0x7fffffff) {
+      pot3d_set_error("pot3d_fno_permute: too many elements");
+      return POT3D_ERR_ARG;
+    }
+    const long long os[4] = {a.od[1] * a.od[2] * a.od[3], a.od[2] * a.od[3], a.od[3], 1};
+    const TileArgs t{in,      out,     a.is[3],        a.is[u],         a.is[v],           os[q],
+                     os[u],   os[v],   a.ie[q],        a.ie[3],         a.ie[u],           a.ie[v],
+                     a.od[q], a.od[3], (unsigned)t3,   (unsigned)tq,    (unsigned)a.od[v], add};
+    const unsigned blocks = (unsigned)nb;
+    if (in_dt == DT_F32 && out_dt == DT_F32)
+      k_permute_tile<float, float><<<blocks, 256, 0, s>>>(t);
+    else if (in_dt == DT_F32)
+      k_permute_tile<float, __nv_bfloat16><<<blocks, 256, 0, s>>>(t);
+    else if (out_dt == DT_F32)
+      k_permute_tile<__nv_bfloat16, float><<<blocks, 256, 0, s>>>(t);
+    else
+      k_permute_tile<__nv_bfloat16, __nv_bfloat16><<<blocks, 256, 0, s>>>(t);
+  }
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_permute");
+}
+
+extern "C" int pot3d_fno_spec_act(float *pre, const void *spec, int B, int W, int nph, int nth, int Pth, int act,
+                                  int keep, void *vout, void *stream) {
+  const long long blocks = (long long)B * nph * ((nth + 31) / 32);
+  if (B < 1 || W < 1 || W > 64 || nph < 1 || nth < 1 || Pth < nth || blocks > 0x7fffffff) {
+    pot3d_set_error("pot3d_fno_spec_act: bad sizes");
+    return POT3D_ERR_ARG;
+  }
+  k_spec_act<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
+      pre, reinterpret_cast<const __nv_bfloat16 *>(spec), W, nph, nth, Pth, act, keep,
+      reinterpret_cast<__nv_bfloat16 *>(vout));
+  return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_spec_act");
 }
 
 extern "C" int pot3d_fno_gelu(const float *pre, long long M, int C, int ldp, const void *grad, int g_dt, int ldg,
@@ -225,7 +394,7 @@ extern "C" int pot3d_fno_gelu(const float *pre, long long M, int C, int ldp, con
     pot3d_set_error("pot3d_fno_gelu: bad sizes");
     return POT3D_ERR_ARG;
   }
-  k_gelu<<<grid_for(M * ldo), 256, 0, (cudaStream_t)stream>>>(pre, M, C, ldp, grad, g_dt, ldg, out, out_dt, ldo,
+  k_gelu<<<grid_for(M * 32), 256, 0, (cudaStream_t)stream>>>(pre, M, C, ldp, grad, g_dt, ldg, out, out_dt, ldo,
                                                                backward);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_gelu");
 }
@@ -237,7 +406,7 @@ extern "C" int pot3d_fno_colsum(const float *in, long long M, int C, int ld, flo
     pot3d_set_error("pot3d_fno_colsum: bad sizes or scratch too small");
     return POT3D_ERR_ARG;
   }
-  k_colsum<<<dim3(nb, C), 256, 0, (cudaStream_t)stream>>>(in, M, C, ld, scratch);
+  k_colsum<<<dim3(nb, (C + 31) / 32), 32 * CS_ROWS, 0, (cudaStream_t)stream>>>(in, M, C, ld, scratch);
   k_colsum_final<<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>(scratch, nb, C, out, add);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_colsum");
 }
@@ -248,7 +417,31 @@ extern "C" int pot3d_fno_relmse(const float *pred, int ldp, const void *tgt, int
     pot3d_set_error("pot3d_fno_relmse: bad sizes");
     return POT3D_ERR_ARG;
   }
-  k_relmse<<<nbatch, 256, 0, (cudaStream_t)stream>>>(pred, ldp, tgt, t_dt, npos, R, scale, grad, loss);
+  float *ws = nullptr;
+  cudaStream_t s = (cudaStream_t)stream;
+  const size_t bytes = sizeof(float) * (size_t)pot3d_fno_relmse_scratch(nbatch);
+  int st = pot3d_cuda_status(cudaMallocAsync((void **)&ws, bytes, s), "cudaMallocAsync(relmse)");
+  if (st) return st;
+  st = pot3d_fno_relmse_ws(pred, ldp, tgt, t_dt, nbatch, npos, R, scale, grad, loss, ws, stream);
+  const int fst = pot3d_cuda_status(cudaFreeAsync(ws, s), "cudaFreeAsync(relmse)");
+  return st ? st : fst;
+}
+
+extern "C" int pot3d_fno_relmse_scratch(int nbatch) { return nbatch * (2 * RM_BLOCKS + 1); }
+
+extern "C" int pot3d_fno_relmse_ws(const float *pred, int ldp, const void *tgt, int t_dt, int nbatch, long long npos,
+                                   int R, float scale, float *grad, float *loss, float *ws, void *stream) {
+  if (nbatch < 1 || nbatch > 65535 || npos < 1 || R < 1 || ldp < R || !ws) {
+    pot3d_set_error("pot3d_fno_relmse: bad sizes");
+    return POT3D_ERR_ARG;
+  }
+  cudaStream_t s = (cudaStream_t)stream;
+  float *part = ws, *den = ws + (size_t)nbatch * 2 * RM_BLOCKS;
+  k_relmse_part<<<dim3(RM_BLOCKS, nbatch), 256, 0, s>>>(pred, ldp, tgt, t_dt, npos, R, part);
+  k_relmse_sum<<<nbatch, 32, 0, s>>>(part, den, loss);
+  const long long nb = (npos + RM_POS - 1) / RM_POS;
+  k_relmse_grad<<<dim3((unsigned)(nb < 148 * 16 ? nb : 148 * 16), nbatch), 256, 0, s>>>(pred, ldp, tgt, t_dt, npos, R,
+                                                                                       scale, den, grad);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_relmse");
 }
 
@@ -270,8 +463,9 @@ extern "C" int pot3d_fno_inputs(const float *br0n, const float *consts, long lon
     pot3d_set_error("pot3d_fno_inputs: bad sizes");
     return POT3D_ERR_ARG;
   }
-  k_inputs<<<grid_for(B * npos * 64), 256, 0, (cudaStream_t)stream>>>(br0n, consts, B, npos,
-                                                                     reinterpret_cast<__nv_bfloat16 *>(x));
+  k_inputs<<<grid_for(B * npos * 8), 256, 0, (cudaStream_t)stream>>>(br0n, consts, B, npos,
+                                                                    reinterpret_cast<__nv_bfloat16 *>(x),
+                                                                    (reinterpret_cast<uintptr_t>(x) & 15) == 0);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_inputs");
 }
 
@@ -279,33 +473,32 @@ namespace {
 // x[b][pos * R + i] = sigma[b] * out[b][pos][i], i < R: the network output
 // (FP32, Rp channels per position) cropped to the radial levels and scaled
 // back to the solver's packed FP64 layout (positions (phi, theta), r fastest).
-__global__ void k_guess(const float *__restrict__ out, long long B, long long npos, int Rp, int R,
-                        const double *__restrict__ sigma, double *__restrict__ x) {
-  const long long n = B * npos * R;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % R);
-    const long long bp = t / R;  // b * npos + pos
-    const long long b = bp / npos;
-    x[t] = (double)out[bp * Rp + i] * sigma[b];
+__global__ void __launch_bounds__(256) k_guess(const float *__restrict__ out, long long B, long long npos, int Rp,
+                                               int R, const double *__restrict__ sigma, double *__restrict__ x) {
+  const int lane = threadIdx.x & 31;
+  for (long long bp = blockIdx.x * 8LL + (threadIdx.x >> 5); bp < B * npos; bp += gridDim.x * 8LL) {
+    const double sg = sigma[bp / npos];
+    for (int i = lane; i < R; i += 32) x[bp * R + i] = (double)out[bp * Rp + i] * sg;
   }
 }
 // The same with the radial levels resampled: the network's Rs levels (those
 // of the mesh it was trained on) interpolated linearly onto the solver's R
 // levels, level i from source levels idx[i] and idx[i]+1 with weight w[i]
 // (outside [0, 1] at the ends: linear extrapolation).
-__global__ void k_guess_resampled(const float *__restrict__ out, long long B, long long npos, int Rp,
-                                  const int *__restrict__ idx, const double *__restrict__ w, int R,
-                                  const double *__restrict__ sigma, double *__restrict__ x) {
-  const long long n = B * npos * R;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % R);
-    const long long bp = t / R;  // b * npos + pos
-    const long long b = bp / npos;
-    const float *o = out + bp * Rp + idx[i];
-    const double lo = (double)o[0], hi = (double)o[1];
-    x[t] = fma(w[i], hi - lo, lo) * sigma[b];
+// A warp a position: the levels' indices and weights stay in L1.
+__global__ void __launch_bounds__(256) k_guess_resampled(const float *__restrict__ out, long long B, long long npos,
+                                                         int Rp, const int *__restrict__ idx,
+                                                         const double *__restrict__ w, int R,
+                                                         const double *__restrict__ sigma, double *__restrict__ x) {
+  const int lane = threadIdx.x & 31;
+  for (long long bp = blockIdx.x * 8LL + (threadIdx.x >> 5); bp < B * npos; bp += gridDim.x * 8LL) {
+    const double sg = sigma[bp / npos];
+#pragma unroll 4
+    for (int i = lane; i < R; i += 32) {
+      const float *o = out + bp * Rp + idx[i];
+      const double lo = (double)o[0], hi = (double)o[1];
+      x[bp * R + i] = fma(w[i], hi - lo, lo) * sg;
+    }
   }
 }
 }  // namespace
@@ -317,7 +510,7 @@ extern "C" int pot3d_fno_guess_resampled(const float *out, long long B, long lon
     pot3d_set_error("pot3d_fno_guess_resampled: bad sizes");
     return POT3D_ERR_ARG;
   }
-  k_guess_resampled<<<grid_for(B * npos * R), 256, 0, (cudaStream_t)stream>>>(out, B, npos, Rp, idx, w, R, sigma,
+  k_guess_resampled<<<grid_for(B * npos * 32), 256, 0, (cudaStream_t)stream>>>(out, B, npos, Rp, idx, w, R, sigma,
                                                                               x);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_guess_resampled");
 }
@@ -328,6 +521,6 @@ extern "C" int pot3d_fno_guess(const float *out, long long B, long long npos, in
     pot3d_set_error("pot3d_fno_guess: bad sizes");
     return POT3D_ERR_ARG;
   }
-  k_guess<<<grid_for(B * npos * R), 256, 0, (cudaStream_t)stream>>>(out, B, npos, Rp, R, sigma, x);
+  k_guess<<<grid_for(B * npos * 32), 256, 0, (cudaStream_t)stream>>>(out, B, npos, Rp, R, sigma, x);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_guess");
 }

@@ -9,7 +9,14 @@
 // four-stage shared-memory ring with 3-D TMA loads (128-byte swizzle, no
 // multicast) and issues tcgen05.mma (M=128, N=BN, K=16 per instruction)
 // whose completion is signalled to mbarriers by tcgen05.commit; all four
-// warps then read their 32 TMEM lanes with tcgen05.ld for the epilogue.
+// warps then read their 32 TMEM lanes with tcgen05.ld for the epilogue, which
+// turns the rows through shared memory so that they leave as whole lines.
+// The operator's products are a few K steps deep and hundreds of thousands of
+// rows long, so what bounds them is memory: a CTA takes only the stages that
+// its K needs (K = 128: 64 KB, three CTAs an SM instead of one), so that one
+// CTA's epilogue overlaps another's loads.  Its weight gradients are the
+// opposite, one tile of output and K of some 10^5: their K is split over CTAs
+// (pot3d_tc_gemm_ex), the FP32 partial products summed in split order.
 // Every wait is bounded; a timeout sets *err and the kernel still drains and
 // frees its TMEM.
 #include <cuda.h>
@@ -18,7 +25,11 @@
 
 #include <cstdint>
 #include <string>
+#include <type_traits>
 
+#include "../../include/pot3d_learned.h"
+
+#include "fno_math.cuh"
 #include "pot3d_internal.cuh"
 #include "tma.cuh"
 
@@ -101,13 +112,38 @@ struct GemmSmem {
   static constexpr int b_bytes = BN * GK * 2;
   static constexpr int stage = a_bytes + b_bytes;  // multiple of 1024
   static constexpr int total = GSTAGES * stage + 1024;
+  static int bytes(int nk) { return (nk < GSTAGES ? nk : GSTAGES) * stage + 1024; }
 };
+constexpr int EPITCH = 36;  // floats between rows of a warp's 32 x 32 epilogue tile (16-byte rows, no bank conflicts)
+static_assert(4 * 32 * EPITCH * 4 <= GemmSmem<32>::stage, "the epilogue tiles fit one stage");
+
+// Four consecutive outputs of a row.
+__device__ __forceinline__ void store4(float *d, float4 o, int accumulate) {
+  if (accumulate) {
+    const float4 c = *reinterpret_cast<const float4 *>(d);
+    o = make_float4(o.x + c.x, o.y + c.y, o.z + c.z, o.w + c.w);
+  }
+  *reinterpret_cast<float4 *>(d) = o;
+}
+__device__ __forceinline__ void store4(__nv_bfloat16 *d, float4 o, int accumulate) {
+  __nv_bfloat162 *d2 = reinterpret_cast<__nv_bfloat162 *>(d);
+  if (accumulate) {
+    const float2 a = __bfloat1622float2(d2[0]), b = __bfloat1622float2(d2[1]);
+    o = make_float4(o.x + a.x, o.y + a.y, o.z + b.x, o.w + b.y);
+  }
+  const __nv_bfloat162 lo = __float22bfloat162_rn(make_float2(o.x, o.y)),
+                       hi = __float22bfloat162_rn(make_float2(o.z, o.w));
+  uint2 w;
+  w.x = *reinterpret_cast<const uint32_t *>(&lo);
+  w.y = *reinterpret_cast<const uint32_t *>(&hi);
+  *reinterpret_cast<uint2 *>(d) = w;
+}
 
 template <int BN, bool OUT_BF16>
 __global__ void __launch_bounds__(128, 1)
     k_gemm_tc(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, void *D,
               const float *__restrict__ bias, int M, int N, int K, long long ldd, long long bstride_d, int accumulate,
-              int *err) {
+              int act, int vec, int per, int splits, int *err) {
   using S = GemmSmem<BN>;
   extern __shared__ __align__(1024) unsigned char gsm[];
   __shared__ __align__(8) uint64_t full[GSTAGES], empty[GSTAGES], done;
@@ -115,8 +151,9 @@ __global__ void __launch_bounds__(128, 1)
   __shared__ int failed;
   unsigned char *base = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(gsm) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.x * GM, n0 = blockIdx.y * BN, bz = blockIdx.z;
-  const int nk = K / GK;
+  // blockIdx.z: the batch, or split * batch + the batch (each split `per` K steps, its product at batch index z)
+  const int m0 = blockIdx.x * GM, n0 = blockIdx.y * BN, nb = gridDim.z / splits, bz = blockIdx.z % nb;
+  const int kb0 = (blockIdx.z / nb) * per, nk = min(per, K / GK - kb0);
   constexpr uint32_t ncols = BN < 32 ? 32 : BN;
 
   if (warp == 0) tmem_alloc(&tmem_base, ncols);
@@ -139,8 +176,8 @@ __global__ void __launch_bounds__(128, 1)
       const int s = kb % GSTAGES;
       unsigned char *sa = base + s * S::stage;
       mbar_expect_tx(&full[s], S::stage);
-      tma_load_3d(sa, &ta, kb * GK, m0, bz, &full[s]);
-      tma_load_3d(sa + S::a_bytes, &tb, kb * GK, n0, bz, &full[s]);
+      tma_load_3d(sa, &ta, (kb0 + kb) * GK, m0, bz, &full[s]);
+      tma_load_3d(sa + S::a_bytes, &tb, (kb0 + kb) * GK, n0, bz, &full[s]);
     };
     int issued = 0;
     for (; issued < GSTAGES && issued < nk; issued++) load(issued);
@@ -181,26 +218,40 @@ __global__ void __launch_bounds__(128, 1)
   if (!got && lane == 0) atomicExch(err, 1);
   __syncthreads();
   if (got && !failed) {
-    const int row = m0 + warp * 32 + lane;
-    for (int c0 = 0; c0 < BN; c0 += 32) {
+    using T = typename std::conditional<OUT_BF16, __nv_bfloat16, float>::type;
+    T *out = reinterpret_cast<T *>(D) + (long long)blockIdx.z * bstride_d;
+    float *tile = reinterpret_cast<float *>(base) + warp * 32 * EPITCH;  // the MMAs have read the stages
+    for (int c0 = 0; c0 < BN && n0 + c0 < N; c0 += 32) {
       float v[32];
       tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-      if (row < M) {
-        const long long off = (long long)bz * bstride_d + (long long)row * ldd;
+#pragma unroll
+      for (int q = 0; q < 32; q++) {
+        if (bias && n0 + c0 + q < N) v[q] += bias[n0 + c0 + q];
+        if (act) v[q] = gelu_f(v[q]);
+      }
+      if (vec) {
+#pragma unroll
+        for (int q = 0; q < 32; q += 4)
+          *reinterpret_cast<float4 *>(tile + lane * EPITCH + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+        __syncwarp();
+        const int col = n0 + c0 + (lane & 7) * 4;  // eight lanes a row, four rows at once
+#pragma unroll
+        for (int r = lane >> 3; r < 32; r += 4) {
+          const int row = m0 + warp * 32 + r;
+          if (row < M && col < N)
+            store4(out + (long long)row * ldd + col, *reinterpret_cast<const float4 *>(tile + r * EPITCH + (lane & 7) * 4),
+                   accumulate);
+        }
+        __syncwarp();
+      } else {
+        const int row = m0 + warp * 32 + lane;
 #pragma unroll
         for (int q = 0; q < 32; q++) {
           const int col = n0 + c0 + q;
-          if (col < N) {
-            float o = v[q] + (bias ? bias[col] : 0.0f);
-            if (OUT_BF16) {
-              __nv_bfloat16 *d = reinterpret_cast<__nv_bfloat16 *>(D) + off + col;
-              if (accumulate) o += __bfloat162float(*d);
-              *d = __float2bfloat16_rn(o);
-            } else {
-              float *d = reinterpret_cast<float *>(D) + off + col;
-              if (accumulate) o += *d;
-              *d = o;
-            }
+          if (row < M && col < N) {
+            T *dst = out + (long long)row * ldd + col;
+            const float o = accumulate ? v[q] + (float)*dst : v[q];
+            *dst = (T)o;
           }
         }
       }
@@ -250,7 +301,7 @@ int map_bf16(CUtensorMap *m, const void *ptr, int batch, int rows, int K, int bo
 
 template <int BN, bool OB>
 int launch(const CUtensorMap &ta, const CUtensorMap &tb, void *D, const float *bias, int batch, int M, int N, int K,
-           long long ldd, long long bsd, int acc, int *err, cudaStream_t st) {
+           long long ldd, long long bsd, int acc, int act, int splits, int *err, cudaStream_t st) {
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(k_gemm_tc<BN, OB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -258,8 +309,12 @@ int launch(const CUtensorMap &ta, const CUtensorMap &tb, void *D, const float *b
     if (e != cudaSuccess) return pot3d_cuda_status(e, "cudaFuncSetAttribute(k_gemm_tc)");
     attr = true;
   }
-  dim3 grid((M + GM - 1) / GM, (N + BN - 1) / BN, batch);
-  k_gemm_tc<BN, OB><<<grid, 128, GemmSmem<BN>::total, st>>>(ta, tb, D, bias, M, N, K, ldd, bsd, acc, err);
+  dim3 grid((M + GM - 1) / GM, (N + BN - 1) / BN, batch * splits);
+  const int per = (K / GK + splits - 1) / splits;
+  // four outputs of a row at once: 16 (FP32) or 8 (BF16) bytes
+  const int vec = ldd % 4 == 0 && bsd % 4 == 0 && (reinterpret_cast<uintptr_t>(D) & (OB ? 7 : 15)) == 0;
+  k_gemm_tc<BN, OB><<<grid, 128, GemmSmem<BN>::bytes(per), st>>>(ta, tb, D, bias, M, N, K, ldd, bsd, acc, act, vec, per,
+                                                                 splits, err);
   return pot3d_cuda_status(cudaGetLastError(), "k_gemm_tc");
 }
 
@@ -273,8 +328,52 @@ int launch(const CUtensorMap &ta, const CUtensorMap &tb, void *D, const float *b
 extern "C" int pot3d_tc_gemm(const void *A, const void *B, void *D, const float *bias, int batch, int M, int N,
                              int K, long long ldd, long long bstride_d, int accumulate, int out_bf16, int *err,
                              void *stream) {
+  return pot3d_tc_gemm_ex(A, B, D, bias, batch, M, N, K, ldd, bstride_d, accumulate, out_bf16, 0, 1, nullptr, err,
+                          stream);
+}
+
+namespace {
+// D (+)= the splits' partial products (+ bias), summed in a fixed order: a
+// block takes 32 outputs, 32 threads an output.
+__global__ void __launch_bounds__(1024) k_splitk_sum(const float *__restrict__ ws, int splits, long long mn, int M, int N,
+                                                     int batch, const float *__restrict__ bias, float *__restrict__ D,
+                                                     long long ldd, long long bstride_d, int accumulate, int act) {
+  const long long n = mn * batch, t = blockIdx.x * 32LL + (threadIdx.x & 31);
+  const int y = threadIdx.x >> 5;
+  float s = 0.0f;
+  if (t < n) {
+#pragma unroll 4
+    for (int q = y; q < splits; q += 32) s += ws[q * n + t];
+  }
+  __shared__ float red[32][32];
+  red[y][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (y == 0 && t < n) {
+    s = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 32; q++) s += red[q][threadIdx.x];
+    const int col = (int)(t % N);
+    const long long row = t / N % M, b = t / mn;
+    if (bias) s += bias[col];
+    if (act) s = gelu_f(s);
+    float *d = D + b * bstride_d + row * ldd + col;
+    *d = accumulate ? *d + s : s;
+  }
+}
+}  // namespace
+
+// The same with a GELU of the result (act; not with accumulate) and, for an
+// FP32 output, K split over `splits` CTAs per tile: ws holds splits * batch *
+// M * N floats.
+extern "C" int pot3d_tc_gemm_ex(const void *A, const void *B, void *D, const float *bias, int batch, int M, int N,
+                                int K, long long ldd, long long bstride_d, int accumulate, int out_bf16, int act,
+                                int splits, float *ws, int *err, void *stream) {
   if (!A || !B || !D || !err || batch < 1 || M < 1 || N < 16 || K < 64 || K % 64 || N % 16 || ldd < N) {
     pot3d_set_error("pot3d_tc_gemm: K must be a positive multiple of 64, N a multiple of 16, ldd >= N");
+    return POT3D_ERR_ARG;
+  }
+  if ((act && accumulate) || splits < 1 || (splits > 1 && (!ws || out_bf16))) {
+    pot3d_set_error("pot3d_tc_gemm_ex: act excludes accumulate; splits need a workspace and an FP32 output");
     return POT3D_ERR_ARG;
   }
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) {
@@ -287,13 +386,25 @@ extern "C" int pot3d_tc_gemm(const void *A, const void *B, void *D, const float 
   if ((st = map_bf16(&ta, A, batch, M, K, GM))) return st;
   if ((st = map_bf16(&tb, B, batch, N, K, BN))) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-#define POT3D_GEMM_CASE(bn)                                                                                   \
-  if (BN == bn)                                                                                               \
-    return out_bf16 ? launch<bn, true>(ta, tb, D, bias, batch, M, N, K, ldd, bstride_d, accumulate, err, s)   \
-                    : launch<bn, false>(ta, tb, D, bias, batch, M, N, K, ldd, bstride_d, accumulate, err, s);
+  splits = splits > K / GK ? K / GK : splits;
+  splits = (K / GK + (K / GK + splits - 1) / splits - 1) / ((K / GK + splits - 1) / splits);  // none empty
+  const bool split = splits > 1;
+  const long long mn = (long long)M * N;
+  void *out = split ? ws : D;
+  const float *b1 = split ? nullptr : bias;
+  const long long ld1 = split ? N : ldd, bs1 = split ? mn : bstride_d;
+  const int acc1 = split ? 0 : accumulate, act1 = split ? 0 : act;
+#define POT3D_GEMM_CASE(bn)                                                                                     \
+  if (BN == bn)                                                                                                 \
+    st = out_bf16 ? launch<bn, true>(ta, tb, out, b1, batch, M, N, K, ld1, bs1, acc1, act1, splits, err, s)     \
+                  : launch<bn, false>(ta, tb, out, b1, batch, M, N, K, ld1, bs1, acc1, act1, splits, err, s);
   POT3D_GEMM_CASE(32)
   POT3D_GEMM_CASE(64)
   POT3D_GEMM_CASE(128)
 #undef POT3D_GEMM_CASE
-  return POT3D_ERR_ARG;
+  if (st || !split) return st;
+  const long long n = mn * batch;
+  k_splitk_sum<<<(unsigned)((n + 31) / 32), 1024, 0, s>>>(ws, splits, mn, M, N, batch, bias,
+                                                          reinterpret_cast<float *>(D), ldd, bstride_d, accumulate, act);
+  return pot3d_cuda_status(cudaGetLastError(), "k_splitk_sum");
 }

@@ -52,7 +52,8 @@ def _L():
                                         C.c_int, vp]
         L.pot3d_fno_gelu.argtypes = [vp, ll, C.c_int, C.c_int, vp, C.c_int, C.c_int, vp, C.c_int, C.c_int, C.c_int, vp]
         L.pot3d_fno_colsum.argtypes = [vp, ll, C.c_int, C.c_int, vp, C.c_int, vp, C.c_int, vp]
-        L.pot3d_fno_relmse.argtypes = [vp, C.c_int, vp, C.c_int, C.c_int, ll, C.c_int, C.c_float, vp, vp, vp]
+        L.pot3d_fno_relmse_ws.argtypes = [vp, C.c_int, vp, C.c_int, C.c_int, ll, C.c_int, C.c_float, vp, vp, vp, vp]
+        L.pot3d_fno_spec_act.argtypes = [vp, vp] + [C.c_int] * 7 + [vp, vp]
         L.pot3d_fno_adam.argtypes = [vp, vp, vp, vp, vp, ll, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int, vp]
         L.pot3d_fno_inputs.argtypes = [vp, vp, ll, ll, vp, vp]
         L.pot3d_fno_guess.argtypes = [vp, ll, ll, C.c_int, C.c_int, vp, vp, vp]
@@ -101,6 +102,16 @@ def act(pre, C_, ldp, out, ldo, mode, grad=None, ldg=0):
                                    C.c_void_p(grad.data_ptr()) if grad is not None else None,
                                    _dt(grad) if grad is not None else 0, ldg, C.c_void_p(out.data_ptr()), _dt(out),
                                    ldo, bwd, _stream()))
+    return out
+
+
+def spec_act(pre, spec, B, W, nph, nth, Pth, gelu, keep):
+    """The next layer's input [M, 64] (BF16): pre + the spectral term (and its
+    GELU); with keep, pre becomes the sum (the backward pass reads it)."""
+    out = new((B * nph * nth, 64), "bf16")
+    _count()
+    _lib.check(_L().pot3d_fno_spec_act(C.c_void_p(pre.data_ptr()), C.c_void_p(spec.data_ptr()), B, W, nph, nth, Pth,
+                                       int(gelu), int(keep), C.c_void_p(out.data_ptr()), _stream()))
     return out
 
 
@@ -255,13 +266,15 @@ class FNO:
             last = l == self.nl - 1
             st = self._spectral(v, B, cache, l)
             pre = tc_gemm(v, self.pb[f"W{l}"], bias=self.p[f"b{l}"])  # [M, 32]
-            permute(st, (B, W_, g.nph, self.Pth), pre, (B, g.nph, g.nth, W_), (0, 2, 3, 1), add=True)
             if keep:
                 cache[f"v{l}"] = v
                 cache[f"pre{l}"] = pre
-            v = act(pre, W_, W_, new((M, 64), "bf16"), 64, "copy" if last else "gelu")
-        hpre = tc_gemm(v, self.pb["Q1"], bias=self.p["bq1"])
-        h = act(hpre, self.hidden, self.hidden, new((M, self.hidden), "bf16"), self.hidden, "gelu")
+            v = spec_act(pre, st, B, W_, g.nph, g.nth, self.Pth, not last, keep)
+        if keep:
+            hpre = tc_gemm(v, self.pb["Q1"], bias=self.p["bq1"])
+            h = act(hpre, self.hidden, self.hidden, new((M, self.hidden), "bf16"), self.hidden, "gelu")
+        else:
+            h = tc_gemm(v, self.pb["Q1"], bias=self.p["bq1"], out_dtype=_bf(), act="gelu")
         out = tc_gemm(h, self.pb["Q2"], bias=self.p["bq2"])
         if keep:
             cache.update(vL=v, hpre=hpre, h=h)
@@ -355,10 +368,12 @@ class FNO:
         npos = self.g.nph * self.g.nth
         grad = torch.empty_like(out)
         loss = new((B,), "f32")
-        _count()
-        _lib.check(_L().pot3d_fno_relmse(C.c_void_p(out.data_ptr()), self.Rp, C.c_void_p(target.data_ptr()),
-                                         _dt(target), B, npos, self.g.R, 1.0 / B, C.c_void_p(grad.data_ptr()),
-                                         C.c_void_p(loss.data_ptr()), _stream()))
+        ws = new((_L().pot3d_fno_relmse_scratch(B),), "f32")
+        for _ in range(3):
+            _count()
+        _lib.check(_L().pot3d_fno_relmse_ws(C.c_void_p(out.data_ptr()), self.Rp, C.c_void_p(target.data_ptr()),
+                                            _dt(target), B, npos, self.g.R, 1.0 / B, C.c_void_p(grad.data_ptr()),
+                                            C.c_void_p(loss.data_ptr()), C.c_void_p(ws.data_ptr()), _stream()))
         return loss, grad
 
     def adam_step(self, grads, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):

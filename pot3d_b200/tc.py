@@ -18,10 +18,9 @@ LAUNCHES = [0]
 
 def _fn():
     L = _lib.lib()
-    f = L.pot3d_tc_gemm
+    f = L.pot3d_tc_gemm_ex
     if not getattr(f, "_typed", False):
-        f.argtypes = [C.c_void_p] * 4 + [C.c_int] * 4 + [C.c_longlong, C.c_longlong, C.c_int, C.c_int, C.c_void_p,
-                                                          C.c_void_p]
+        f.argtypes = [C.c_void_p] * 4 + [C.c_int] * 4 + [C.c_longlong, C.c_longlong] + [C.c_int] * 4 + [C.c_void_p] * 3
         f.restype = C.c_int
         f._typed = True
     return f
@@ -35,9 +34,20 @@ def _err_flag(device):
     return _err[key]
 
 
-def tc_gemm(A, B, bias=None, out=None, out_dtype=None, ldd=None, accumulate=False, n=None):
+def k_splits(batch, M, N, K):
+    """Blocks that share the K of one output tile: a product with fewer tiles
+    than half the SMs and a K of 64 or more steps is split so that about two
+    blocks an SM have work, each with at least 8 steps."""
+    tile_n = 32 if N <= 32 else 64 if N <= 64 else 128
+    tiles = batch * -(-M // 128) * -(-N // tile_n)
+    steps = K // 64
+    return max(1, min(steps // 8, -(-296 // tiles))) if tiles <= 74 and steps >= 64 else 1
+
+
+def tc_gemm(A, B, bias=None, out=None, out_dtype=None, ldd=None, accumulate=False, n=None, act=None):
     """out[b, m, :n] (+)= A[b] @ B[b]^T (+ bias).  `out` may be wider than N
-    (row stride ldd, e.g. a zero-padded channel buffer)."""
+    (row stride ldd, e.g. a zero-padded channel buffer).  act "gelu" applies
+    the activation to the result."""
     import torch
     squeeze = A.dim() == 2
     if squeeze:
@@ -57,13 +67,15 @@ def tc_gemm(A, B, bias=None, out=None, out_dtype=None, ldd=None, accumulate=Fals
     ldd = out.shape[-1] if ldd is None else ldd
     assert ldd >= N and out.shape[-1] == ldd
     err = _err_flag(A.device)
+    splits = k_splits(bsz, M, N, K) if out.dtype == torch.float32 else 1
+    ws = torch.empty(splits * bsz * M * N, dtype=torch.float32, device=A.device) if splits > 1 else None
     stream = torch.cuda.current_stream(A.device).cuda_stream
     rc = _fn()(C.c_void_p(A.data_ptr()), C.c_void_p(B.data_ptr()), C.c_void_p(out.data_ptr()),
                C.c_void_p(bias.data_ptr()) if bias is not None else None, bsz, M, N, K, ldd, M * ldd,
-               1 if accumulate else 0, 1 if out.dtype == torch.bfloat16 else 0, C.c_void_p(err.data_ptr()),
-               C.c_void_p(stream))
+               1 if accumulate else 0, 1 if out.dtype == torch.bfloat16 else 0, 1 if act == "gelu" else 0, splits,
+               C.c_void_p(ws.data_ptr()) if ws is not None else None, C.c_void_p(err.data_ptr()), C.c_void_p(stream))
     _lib.check(rc)
-    LAUNCHES[0] += 1
+    LAUNCHES[0] += 2 if splits > 1 else 1
     return out[0] if squeeze else out
 
 

@@ -1,0 +1,114 @@
+"""Kernels of the learned operator at the sizes where they can go wrong:
+permutations through shared-memory tiles (remainders in both tiled axes,
+padding, cropping, accumulation), products with a split K, a strided or
+unaligned output and the GELU epilogue, the fused layer sum, column sums and
+the loss over many blocks.  References are torch on the same inputs in FP64;
+permutations are exact, FP32 sums of n terms are held to 4 sqrt(n) roundings
+of the sum of magnitudes, BF16 outputs to their rounding."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+EPS32, EPS16 = 2.0 ** -24, 2.0 ** -8
+
+
+def _t(shape, cuda, seed=0, dtype=None):
+    import torch
+    g = torch.Generator(device=cuda).manual_seed(seed)
+    x = torch.randn(shape, device=cuda, generator=g)
+    return x.to(dtype) if dtype else x
+
+
+@pytest.mark.parametrize("perm", [(0, 1, 3, 2), (0, 3, 1, 2), (0, 2, 3, 1), (2, 3, 0, 1), (0, 1, 2, 3), (3, 0, 1, 2)])
+@pytest.mark.parametrize("dims", [(2, 3, 130, 65), (1, 2, 1, 33), (3, 1, 257, 16)])
+def test_permute_pads_crops_and_adds(cuda, perm, dims):
+    import torch
+    from pot3d_b200.fno import permute
+    for src, dst, add in (("bf16", "bf16", False), ("f32", "bf16", False), ("bf16", "f32", True), ("f32", "f32", False)):
+        dt = {"bf16": torch.bfloat16, "f32": torch.float32}
+        x = _t(dims, cuda, 1, dt[src])
+        out_dims = [dims[p] for p in perm]
+        out_dims[3] += 5      # padded
+        out_dims[2] = max(1, out_dims[2] - 1)  # cropped
+        out = _t(out_dims, cuda, 2, dt[dst]) if add else torch.full(out_dims, 7.0, device=cuda, dtype=dt[dst])
+        ref = x.permute(*perm)[:, :, :out_dims[2]].float()
+        ref = torch.nn.functional.pad(ref, (0, 5))
+        ref = (out.float() + ref if add else ref).to(dt[dst])
+        permute(x, dims, out, out_dims, perm, add=add)
+        assert torch.equal(out, ref), (src, dst, add)
+
+
+@pytest.mark.parametrize("b,m,n,k", [(1, 32, 64, 64 * 67), (1, 128, 128, 64 * 300), (1, 130, 16, 64 * 64),
+                                     (2, 32, 32, 64 * 65), (1, 1000, 48, 64)])
+def test_gemm_split_k_strides_and_act(cuda, b, m, n, k):
+    import torch
+    from pot3d_b200.tc import check_errors, k_splits, tc_gemm
+    A, B, bias = _t((b, m, k), cuda, 3, torch.bfloat16), _t((b, n, k), cuda, 4, torch.bfloat16), _t((n,), cuda, 5)
+    ref = A.double() @ B.double().transpose(1, 2) + bias.double()
+    mag = A.double().abs() @ B.double().abs().transpose(1, 2) + bias.double().abs()
+    tol = 4 * EPS32 * np.sqrt(k) * mag
+    splits = k_splits(b, m, n, k)
+    assert (splits > 1) == (k >= 64 * 64)
+    assert bool(((tc_gemm(A, B, bias=bias).double() - ref).abs() <= tol).all())
+    acc = _t((b, m, n), cuda, 6)
+    got = tc_gemm(A, B, bias=bias, out=acc.clone(), accumulate=True)
+    assert bool(((got.double() - ref - acc.double()).abs() <= tol + EPS32 * (ref + acc.double()).abs()).all())
+    g = torch.nn.functional.gelu(ref, approximate="tanh")
+    assert bool(((tc_gemm(A, B, bias=bias, act="gelu").double() - g).abs() <= 2 * tol + 16 * EPS32 * g.abs()).all())
+    wide = torch.full((b, m, n + 3), 7.0, device=cuda)  # a row stride that rules out vector stores
+    tc_gemm(A, B, bias=bias, out=wide, ldd=n + 3)
+    assert bool(((wide[..., :n].double() - ref).abs() <= tol).all()) and bool((wide[..., n:] == 7.0).all())
+    if splits == 1:  # the BF16 output is the FP32 one rounded
+        assert torch.equal(tc_gemm(A, B, bias=bias, out_dtype=torch.bfloat16), tc_gemm(A, B, bias=bias).bfloat16())
+    check_errors()
+
+
+@pytest.mark.parametrize("b,w,nph,nth", [(1, 32, 3, 33), (2, 17, 5, 31), (1, 64, 2, 96)])
+def test_spec_act(cuda, b, w, nph, nth):
+    import torch
+    from pot3d_b200.fno import spec_act
+    pth = (nth + 63) // 64 * 64
+    pre = _t((b * nph * nth, w), cuda, 7)
+    spec = _t((b, w, nph, pth), cuda, 8, torch.bfloat16)
+    s = pre + spec[..., :nth].permute(0, 2, 3, 1).reshape(-1, w).float()
+    for gelu in (False, True):
+        p = pre.clone()
+        v = spec_act(p, spec, b, w, nph, nth, pth, gelu, keep=gelu)
+        assert torch.equal(p, s if gelu else pre)
+        ref = torch.nn.functional.gelu(s.double(), approximate="tanh") if gelu else s.double()
+        assert bool(((v[:, :w].double() - ref).abs() <= (EPS16 + 32 * EPS32) * ref.abs() + 1e-7).all())
+        assert not v[:, w:].any()
+
+
+@pytest.mark.parametrize("b,npos,R,ldp", [(1, 1, 1, 64), (3, 2049, 125, 128), (2, 70000, 61, 64)])
+def test_relmse_and_colsum(cuda, b, npos, R, ldp):
+    import torch
+    from pot3d_b200 import _lib
+    from pot3d_b200.fno import _L, colsum, new
+    pred, tgt = _t((b, npos, ldp), cuda, 9), _t((b, npos, R), cuda, 10, torch.bfloat16)
+    d = pred[..., :R].double() - tgt.double()
+    den = tgt.double().square().sum((1, 2))
+    loss = d.square().sum((1, 2)) / den
+    gref = torch.nn.functional.pad(2.0 * 0.25 * d / den.view(-1, 1, 1), (0, ldp - R))
+    tol = 8 * EPS32 * np.sqrt(npos * R)
+    L = _L()
+    for scratch in (True, False):
+        grad, got = torch.full_like(pred, 7.0), torch.zeros(b, device=cuda)
+        args = [C.c_void_p(pred.data_ptr()), ldp, C.c_void_p(tgt.data_ptr()), 1, b, C.c_longlong(npos), R,
+                C.c_float(0.25), C.c_void_p(grad.data_ptr()), C.c_void_p(got.data_ptr())]
+        if scratch:
+            ws = new((L.pot3d_fno_relmse_scratch(b),), "f32")
+            _lib.check(L.pot3d_fno_relmse_ws(*args, C.c_void_p(ws.data_ptr()), None))
+        else:
+            _lib.check(L.pot3d_fno_relmse(*args, None))
+        torch.cuda.synchronize()
+        assert bool(((got.double() - loss).abs() <= tol * loss).all())
+        assert bool(((grad.double() - gref).abs() <= (tol + 8 * EPS32) * gref.abs() + 4 * EPS32 * 0.5 / den.view(-1, 1, 1) *
+                     (pred.abs().double().amax() + tgt.abs().double().amax())).all())
+    flat = pred.reshape(-1, ldp)
+    s = colsum(flat, R, ldp, new((R,), "f32"))
+    ref = flat[:, :R].double().sum(0)
+    assert bool(((s.double() - ref).abs() <= 4 * EPS32 * np.sqrt(b * npos) * flat[:, :R].double().abs().sum(0) + 1e-30).all())
