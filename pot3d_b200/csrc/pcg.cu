@@ -176,7 +176,7 @@ struct StencilArgs {
   double *s1p;              // PCG: [2][NRP] ring sums of p (parity buffers)
   SolveState *st;
   double *partials;
-  int xslot1;               // refined ILU(0): 1 + the slot of st->xa that receives alpha (0: none)
+  int xslot1;               // 1 + the slot of st->xa that receives alpha (0: none)
 };
 
 // Shared-memory layout of the TMA-staged stencil.  Each pipeline stage holds
@@ -264,18 +264,6 @@ __device__ __forceinline__ void stencil_body(const StencilMaps &maps, const Geo 
   __shared__ double s1sh[TI];
   __shared__ int abort_flag;
 
-  double beta = 0.0;
-  int par = 0;
-  if (MODE != MODE_AX) {
-    const volatile SolveState *vs = a.st;
-    if (vs->status != ST_RUNNING) {  // uniform: converged or failed
-      // no iteration: the paired x update applies nothing for it
-      if (a.xslot1 && bx == 0 && by == 0 && bz == 0 && threadIdx.x == 0) a.st->xa[a.xslot1 - 1] = 0.0;
-      return;
-    }
-    beta = vs->beta;
-    par = vs->par;
-  }
   double *kfac = reinterpret_cast<double *>(dyn + L::kfac_off);  // [tk][3]
   unsigned char *base = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~uintptr_t(127));
   // p_new ring [PN_SLOTS][BOX_Y][BOX64_X], FP64 in every mode: the FP32 modes
@@ -307,6 +295,42 @@ __device__ __forceinline__ void stencil_body(const StencilMaps &maps, const Geo 
     for (int q = 0; q < L::n32; q++) tma_prefetch_desc(&maps.m32[q]);
   }
   if (tid < TI) s1sh[tid] = 0.0;
+  PtFac f0, f1;
+  auto mesh_factors = [&]() {
+    const int jf = jj + 2;
+    if (rowv) {
+      f0 = pt_fac(m, min(e0, g.nrm2 - 1) + 2, jf);
+      f1 = pt_fac(m, min(e0 + 1, g.nrm2 - 1) + 2, jf);
+    }
+    // dp_i(k-1), dp_i(k), dph(k) of the block's planes, staged once.
+    for (int q = tid; q < k1 - k0; q += NTHR) {
+      const int kf = k0 + q + 2;
+      kfac[3 * q + 0] = m.dp_i[kf - 1];
+      kfac[3 * q + 1] = m.dp_i[kf];
+      kfac[3 * q + 2] = m.dph[kf];
+    }
+  };
+  // The diagonal modes are launched before the kernel they follow has ended
+  // and form the mesh factors meanwhile; the others form them behind the
+  // first loads.
+  constexpr bool EARLY = MODE == MODE_PCG || MODE == MODE_PCG32;
+  if constexpr (EARLY) {
+    mesh_factors();
+    pdl_wait();
+    pdl_trigger();
+  }
+  double beta = 0.0;
+  int par = 0;
+  if (MODE != MODE_AX) {
+    const volatile SolveState *vs = a.st;
+    if (vs->status != ST_RUNNING) {  // uniform: converged or failed
+      // no iteration: the grouped x update applies nothing for it
+      if (a.xslot1 && bx == 0 && by == 0 && bz == 0 && threadIdx.x == 0) a.st->xa[a.xslot1 - 1] = 0.0;
+      return;
+    }
+    beta = vs->beta;
+    par = vs->par;
+  }
   __syncthreads();
 
   const int p_first = k0 - 1;         // planes p_first .. k1 feed the stencil
@@ -341,19 +365,7 @@ __device__ __forceinline__ void stencil_body(const StencilMaps &maps, const Geo 
     }
   }
 
-  const int jf = jj + 2;
-  PtFac f0, f1;
-  if (rowv) {
-    f0 = pt_fac(m, min(e0, g.nrm2 - 1) + 2, jf);
-    f1 = pt_fac(m, min(e0 + 1, g.nrm2 - 1) + 2, jf);
-  }
-  // dp_i(k-1), dp_i(k), dph(k) of the block's planes, staged once.
-  for (int q = tid; q < k1 - k0; q += NTHR) {
-    const int kf = k0 + q + 2;
-    kfac[3 * q + 0] = m.dp_i[kf - 1];
-    kfac[3 * q + 1] = m.dp_i[kf];
-    kfac[3 * q + 2] = m.dph[kf];
-  }
+  if constexpr (!EARLY) mesh_factors();
   __syncthreads();
   const double s1a = south ? s1sh[el] : 0.0, s1b = south ? s1sh[el + 1] : 0.0;
   const double pm = m.pm_r1;
@@ -550,6 +562,8 @@ template <int KIND, bool ZIN, bool R32 = false>
 __device__ __forceinline__ void update_body(const Geo &g, const DevMesh &m, const UpdateArgs &a, const int bx,
                                             const int by, const int bz) {
   __shared__ double red[NTHR / 32];
+  pdl_wait();
+  pdl_trigger();
   const volatile SolveState *vs = a.st;
   if ((KIND == UPD_ITER || KIND == UPD_ZDOT) && vs->status != ST_RUNNING) return;
   const double alpha = (KIND == UPD_ITER) ? vs->alpha : 0.0;
@@ -569,16 +583,18 @@ __device__ __forceinline__ void update_body(const Geo &g, const DevMesh &m, cons
       double2 rv = R32 ? widen2(*reinterpret_cast<const float2 *>(a.r32 + id))
                        : *reinterpret_cast<const double2 *>(a.r + id);
       if (KIND == UPD_ITER) {
-        double2 xv = *reinterpret_cast<const double2 *>(a.x + id);
-        const double2 pv = R32 ? widen2(__ldg(reinterpret_cast<const float2 *>(a.p32 + id)))
-                               : __ldg(reinterpret_cast<const double2 *>(a.p + id));
+        if (a.x) {  // else applied in groups of iterations (k_update_x_group)
+          double2 xv = *reinterpret_cast<const double2 *>(a.x + id);
+          const double2 pv = R32 ? widen2(__ldg(reinterpret_cast<const float2 *>(a.p32 + id)))
+                                 : __ldg(reinterpret_cast<const double2 *>(a.p + id));
+          xv.x = fma(alpha, pv.x, xv.x);
+          xv.y = fma(alpha, pv.y, xv.y);
+          *reinterpret_cast<double2 *>(a.x + id) = xv;
+        }
         const double2 qv = R32 ? widen2(__ldg(reinterpret_cast<const float2 *>(a.q32 + id)))
                                : __ldg(reinterpret_cast<const double2 *>(a.q + id));
-        xv.x = fma(alpha, pv.x, xv.x);
-        xv.y = fma(alpha, pv.y, xv.y);
         rv.x = fma(-alpha, qv.x, rv.x);
         rv.y = fma(-alpha, qv.y, rv.y);
-        *reinterpret_cast<double2 *>(a.x + id) = xv;
         if (R32) {
           const float2 r2 = make_float2((float)rv.x, (float)rv.y);
           *reinterpret_cast<float2 *>(a.r32 + id) = r2;
@@ -685,8 +701,8 @@ __global__ void k_cast_r32(long long n, const double *__restrict__ r, float *__r
 // run).  One fma of FP64 x with the FP32 direction per point and iteration,
 // in iteration order, so x is bit-identical to updating it every iteration,
 // and the solution vector is read and written once per group.  Four
-// unknowns per thread and pass.  Batches use pairs; a single solve groups
-// eight (k_update_x_oct).
+// unknowns per thread and pass.  Batches use pairs; single solves larger groups
+// (k_update_x_group).
 __device__ __forceinline__ void x_pair_body(const Geo &g, const SolveState *st, double *__restrict__ x,
                                             const float *__restrict__ pa, const float *__restrict__ pb, long long t0,
                                             long long stride) {
@@ -715,19 +731,26 @@ __device__ __forceinline__ void x_pair_body(const Geo &g, const SolveState *st, 
     *reinterpret_cast<double2 *>(x + id + 2) = x1;
   }
 }
-// The single solve's groups: eight iterations at once, x += a_0 p_0 + ... +
-// a_7 p_7 in iteration order (the directions of eight consecutive
-// iterations, in the eight rotating buffers), x read and written once per
-// eight iterations: 6 B per unknown and iteration.
+// The single solves' groups: G iterations at once, x += a_0 p_0 + ... +
+// a_{G-1} p_{G-1} in iteration order (the directions of G consecutive
+// iterations, in the rotating buffers), x read and written once per group.
+// With FP32 directions and G = 8 this moves 6 B per unknown and iteration
+// instead of 20, with FP64 directions and G = 4 12 B instead of 24: the
+// 121x181x361 FP64 solve spent 73 us of 134 us an iteration in an update that
+// read and wrote x every time.
+template <typename T, int G>
 struct XDirs {
-  const float *p[X_GROUP];
+  const T *p[G];
 };
-__global__ void __launch_bounds__(NTHR) k_update_x_oct(Geo g, const SolveState *st, double *__restrict__ x,
-                                                       XDirs d) {
-  double a[X_GROUP];
+template <typename T, int G>
+__global__ void __launch_bounds__(NTHR) k_update_x_group(Geo g, const SolveState *st, double *__restrict__ x,
+                                                         XDirs<T, G> d) {
+  pdl_wait();
+  pdl_trigger();
+  double a[G];
   bool any = false;
 #pragma unroll
-  for (int i = 0; i < X_GROUP; i++) {
+  for (int i = 0; i < G; i++) {
     a[i] = *(const volatile double *)&st->xa[i];
     any = any || a[i] != 0.0;
   }
@@ -738,16 +761,25 @@ __global__ void __launch_bounds__(NTHR) k_update_x_oct(Geo g, const SolveState *
     const long long id = 4 * t;
     double2 x0 = *reinterpret_cast<const double2 *>(x + id);
     double2 x1 = *reinterpret_cast<const double2 *>(x + id + 2);
-    float4 v[X_GROUP];
+    double2 v0[G], v1[G];
 #pragma unroll
-    for (int i = 0; i < X_GROUP; i++) v[i] = __ldg(reinterpret_cast<const float4 *>(d.p[i] + id));
+    for (int i = 0; i < G; i++) {
+      if constexpr (sizeof(T) == 4) {
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(d.p[i] + id));
+        v0[i] = make_double2((double)v.x, (double)v.y);
+        v1[i] = make_double2((double)v.z, (double)v.w);
+      } else {
+        v0[i] = __ldg(reinterpret_cast<const double2 *>(d.p[i] + id));
+        v1[i] = __ldg(reinterpret_cast<const double2 *>(d.p[i] + id + 2));
+      }
+    }
 #pragma unroll
-    for (int i = 0; i < X_GROUP; i++) {
+    for (int i = 0; i < G; i++) {
       if (a[i] != 0.0) {
-        x0.x = fma(a[i], (double)v[i].x, x0.x);
-        x0.y = fma(a[i], (double)v[i].y, x0.y);
-        x1.x = fma(a[i], (double)v[i].z, x1.x);
-        x1.y = fma(a[i], (double)v[i].w, x1.y);
+        x0.x = fma(a[i], v0[i].x, x0.x);
+        x0.y = fma(a[i], v0[i].y, x0.y);
+        x1.x = fma(a[i], v1[i].x, x1.x);
+        x1.y = fma(a[i], v1[i].y, x1.y);
       }
     }
     *reinterpret_cast<double2 *>(x + id) = x0;
@@ -810,14 +842,27 @@ __global__ void k_unpack(Geo g, const double *__restrict__ src, double *__restri
   }
 }
 // S1(e) = sum_k x(e, ntm1, k)*dph(k)*pl_i in k order (src/pot3d.F90:5456-5463).
-__global__ void k_ring_south(Geo g, DevMesh m, const double *__restrict__ x, double *__restrict__ s1) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= g.NRP) return;
+// A block takes 32 radial points, its 32 warps 32 planes at a time, so the
+// loads are in flight together; the sum keeps the planes' order.  (One thread
+// walking a radial point's planes alone took 130 us at 127x181x361.)
+__global__ void __launch_bounds__(1024) k_ring_south(Geo g, DevMesh m, const double *__restrict__ x,
+                                                     double *__restrict__ s1) {
+  __shared__ double t[32][33];
+  const int lane = threadIdx.x & 31, y = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
   double s = 0.0;
-  if (e < g.nrm2)
-    for (int kk = 0; kk < g.npm2; kk++)
-      s = s + __dmul_rn(__dmul_rn(x[g.idx(e, g.ntm2 - 1, kk)], m.dph[kk + 2]), m.pl_i);
-  s1[e] = s;
+  for (int k0 = 0; k0 < g.npm2; k0 += 32) {
+    const int kk = k0 + y;
+    t[y][lane] = e < g.nrm2 && kk < g.npm2
+                     ? __dmul_rn(__dmul_rn(x[g.idx(e, g.ntm2 - 1, kk)], m.dph[kk + 2]), m.pl_i)
+                     : 0.0;
+    __syncthreads();
+    if (y == 0) {
+      const int n = min(32, g.npm2 - k0);
+      for (int q = 0; q < n; q++) s = s + t[q][lane];
+    }
+    __syncthreads();
+  }
+  if (y == 0 && e < g.NRP) s1[e] = s;
 }
 // RHS of the boundary trick, src/pot3d.F90:3937-3950: with a zero interior,
 // delsq at i=2 picks up a3*x(1) where x(1) = -br0*dr1 and, for a
@@ -880,6 +925,7 @@ __global__ void k_phi_ring(Geo g, DevMesh m, const double *__restrict__ phi, dou
   if (i > g.nr) return;
   const long long pl = (long long)g.nr * g.nt;
   double s0 = 0.0, s1 = 0.0;
+#pragma unroll 16
   for (int k = 2; k <= g.np - 1; k++) {
     s0 = s0 + __dmul_rn(__dmul_rn(phi[(i - 1) + (long long)g.nr * 1 + pl * (k - 1)], m.dph[k]), m.pl_i);
     s1 = s1 + __dmul_rn(__dmul_rn(phi[(i - 1) + (long long)g.nr * (g.nt - 2) + pl * (k - 1)], m.dph[k]), m.pl_i);
@@ -969,11 +1015,12 @@ __global__ void __launch_bounds__(NTHR) k_getb(Geo g, DevMesh m, const double *_
   }
 }
 __global__ void k_energy_final(const double *__restrict__ part, int nb, double *__restrict__ w) {
-  if (threadIdx.x < 3) {
-    double s = 0.0;
-    for (int b = 0; b < nb; b++) s += part[3 * b + threadIdx.x];
-    w[threadIdx.x] = s;
-  }
+  const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;  // a warp a component; a fixed order
+  double s = 0.0;
+#pragma unroll 8
+  for (int b = lane; b < nb; b += 32) s += part[3 * b + c];
+  s = warp_sum(s);
+  if (lane == 0) w[c] = s;
 }
 // Deterministic dot of two padded vectors (two-stage).
 __global__ void __launch_bounds__(NTHR) k_dot(long long n, const double *__restrict__ x,
@@ -987,11 +1034,11 @@ __global__ void __launch_bounds__(NTHR) k_dot(long long n, const double *__restr
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 __global__ void k_sum_parts(const double *__restrict__ part, int nb, double *__restrict__ out) {
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int b = 0; b < nb; b++) s += part[b];
-    *out = s;
-  }
+  double s = 0.0;  // one warp; a fixed order
+#pragma unroll 8
+  for (int b = threadIdx.x; b < nb; b += 32) s += part[b];
+  s = warp_sum(s);
+  if (threadIdx.x == 0) *out = s;
 }
 __global__ void k_axpy_sub(long long n, const double *__restrict__ q, double *__restrict__ r) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
@@ -1326,16 +1373,11 @@ int Solver::setup(const pot3d_mesh_t *mesh, const double *br0, const double *br1
     const size_t fb = sizeof(float) * (size_t)g.Np;
     if ((st = alloc((void **)&m_p32a, fb)) || (st = alloc((void **)&m_p32b, fb)) || (st = alloc((void **)&m_q32, fb)))
       return st;
-    if (ifprec == 2) {
-      m_p32q[0] = m_p32a;
-      m_p32q[1] = m_p32b;
-      for (int i = 2; i < X_GROUP; i++)
-        if ((st = alloc((void **)&m_p32q[i], fb))) return st;
-    }
     if (ifprec != 2 && (st = alloc((void **)&m_r32, fb))) return st;  // ILU(0) uses the sweeps' r32
     CK(cudaEventCreate(&evm0));
     CK(cudaEventCreate(&evm1));
   }
+  if ((st = x_buffers())) return st;
   CK(cudaStreamSynchronize(stream));
   return POT3D_OK;
 }
@@ -1347,7 +1389,7 @@ int Solver::rhs_padded(double *b) {
 
 // y = A x on padded device vectors with the exact south-pole ring sums.
 int Solver::ax_padded(const double *x, double *y) {
-  k_ring_south<<<(g.NRP + 127) / 128, 128, 0, stream>>>(g, m, x, d_s1);
+  k_ring_south<<<(g.NRP + 31) / 32, 1024, 0, stream>>>(g, m, x, d_s1);
   StencilArgs a{};
   a.x = x;
   a.y = y;
@@ -1392,10 +1434,74 @@ int Solver::unpack(const double *pad_dev, double *ref_dev) {
   return pot3d_cuda_status(cudaGetLastError(), "k_unpack");
 }
 
-// One PCG iteration (src/pot3d.F90:4336-4365).
-int Solver::launch_iteration() {
+// The rotation of direction buffers (xg, xg64).  With the diagonal
+// preconditioner x is updated in groups where the vectors of an iteration
+// outgrow L2 and the update is bound by HBM (121x181x361 FP64: 73 -> 59 us an
+// iteration; 127x181x361 refined: 52 -> 41); below that x stays in L2 and a
+// launch per group costs more than it saves (63x91x181: 11.1 -> 12.9 us).  A
+// rotation that does not fit in memory is left out (groups of two).
+int Solver::x_buffers() {
+  if (batched) return POT3D_OK;  // batches update x in pairs from the two buffers
+  int dev = 0, l2 = 0, st;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+  auto more = [&](void **p, size_t bytes) {
+    const int e = alloc(p, bytes);
+    if (e == POT3D_ERR_NOMEM) cudaGetLastError();
+    return e;
+  };
+  if (precision == POT3D_FP64) {
+    if (ifprec == 2 || 44LL * g.Np <= l2) return POT3D_OK;  // x, r, p, p', q and a_i
+    m_p64q[0] = d_p;
+    m_p64q[1] = d_p2;
+    xg64 = 2;
+    for (int i = 2; i < X_GROUP64; i++) {
+      if ((st = more((void **)&m_p64q[i], sizeof(double) * (size_t)g.Np)) == POT3D_ERR_NOMEM) return POT3D_OK;
+      if (st) return st;
+    }
+    xg64 = X_GROUP64;
+    return POT3D_OK;
+  }
+  m_p32q[0] = m_p32a;
+  m_p32q[1] = m_p32b;
+  if (ifprec != 2 && 28LL * g.Np <= l2) return POT3D_OK;  // x and FP32 r, p, p', q, a_i
+  xg = 2;
+  for (int i = 2; i < X_GROUP; i++) {
+    if ((st = more((void **)&m_p32q[i], sizeof(float) * (size_t)g.Np)) == POT3D_ERR_NOMEM && ifprec != 2) return POT3D_OK;
+    if (st) return st;
+  }
+  xg = X_GROUP;
+  return POT3D_OK;
+}
+
+// x += the n iterations' alpha p, the direction of iteration slot i in buffer
+// (i + 1) % n of the rotation.
+int Solver::launch_x_group(const float *const *dirs32, const double *const *dirs64, int n) {
+  auto go = [&](auto zero, auto gc, const auto *const *dirs) {
+    using T = decltype(zero);
+    constexpr int G = decltype(gc)::value;
+    XDirs<T, G> x;
+    for (int i = 0; i < G; i++) x.p[i] = dirs[(i + 1) % G];
+    if (ifprec != 2) return pot3d_cuda_status(launch_pdl(k_update_x_group<T, G>, dim3(xblocks), dim3(NTHR), 0, stream, g,
+                                                         (const SolveState *)d_state, d_x, x), "k_update_x_group");
+    k_update_x_group<T, G><<<xblocks, NTHR, 0, stream>>>(g, d_state, d_x, x);
+    return pot3d_cuda_status(cudaGetLastError(), "k_update_x_group");
+  };
+  if (dirs32)
+    return n == X_GROUP ? go(0.f, std::integral_constant<int, X_GROUP>{}, dirs32)
+                        : go(0.f, std::integral_constant<int, 2>{}, dirs32);
+  return n == X_GROUP64 ? go(0.0, std::integral_constant<int, X_GROUP64>{}, dirs64)
+                        : go(0.0, std::integral_constant<int, 2>{}, dirs64);
+}
+
+// One PCG iteration (src/pot3d.F90:4336-4365) at position u of a captured graph.
+int Solver::launch_iteration(int u) {
   dim3 grid(g.nit, g.njt, g.nkc);
   dim3 gridu(g.nit, g.njt, g.nkc_u);
+  if (xg64 > 1) {  // the rotation: position u reads buffer u % xg64, writes the next
+    p_cur = m_p64q[u % xg64];
+    p_nxt = m_p64q[(u + 1) % xg64];
+  }
   StencilArgs sa{};
   sa.p_old = p_cur;
   sa.p_new = p_nxt;  // ping-pong: neighbouring tiles still read p_old halos
@@ -1428,12 +1534,18 @@ int Solver::launch_iteration() {
     int st = dilu_sweeps(this, true);
     if (st) return st;
     ua.z32 = dilu_z32(this);
-    k_update<UPD_ZDOT, true><<<gridu, NTHR, 0, stream>>>(g, m, ua);
+    k_update<UPD_ZDOT, true, false><<<gridu, NTHR, 0, stream>>>(g, m, ua);
   } else {
     if ((stm = tensor_map(d_r, true, &mp.m64[1]))) return stm;
     if ((stm = tensor_map(d_ai, false, &mp.m32[0]))) return stm;
-    k_stencil<MODE_PCG><<<grid, NTHR, StageLayout<MODE_PCG>::smem, stream>>>(mp, g, m, sa);
-    k_update<UPD_ITER, false><<<gridu, NTHR, 0, stream>>>(g, m, ua);
+    if (xg64 > 1) {
+      sa.xslot1 = 1 + u % xg64;
+      ua.x = nullptr;
+    }
+    CK(launch_pdl(k_stencil<MODE_PCG>, grid, dim3(NTHR), StageLayout<MODE_PCG>::smem, stream, mp, g, m, sa));
+    CK(launch_pdl(k_update<UPD_ITER, false, false>, gridu, dim3(NTHR), 0, stream, g, m, ua));
+    int st;
+    if (xg64 > 1 && u % xg64 == xg64 - 1 && (st = launch_x_group(nullptr, m_p64q, xg64))) return st;
   }
   std::swap(p_cur, p_nxt);
   return pot3d_cuda_status(cudaGetLastError(), "launch_iteration");
@@ -1514,13 +1626,14 @@ int Solver::cgsolve_padded(bool zero_guess, int ncgmax, double epscg, int *ierr,
     const double est_iter_s = (ifprec == 2 ? 140.0 : 90.0) * (double)g.Np / 5.0e12 + 6e-6;
     int U = (int)std::ceil(0.5e-3 / est_iter_s);
     U = std::max(2, std::min(U, 32));
+    U += U & 1;  // whole groups of the solution update
     if (!graph_exec || graph_U != U || graph_kind != ifprec) {
       if (graph_exec) cudaGraphExecDestroy(graph_exec);
       graph_exec = nullptr;
       cudaGraph_t graph;
       CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-      for (int u = 0; u < 2 * U; u++) {  // even count: p ping-pong returns to d_p
-        st = launch_iteration();
+      for (int u = 0; u < 2 * U; u++) {  // a multiple of 4: the rotation returns to d_p
+        st = launch_iteration(u);
         if (st) {
           cudaStreamEndCapture(stream, &graph);
           if (graph) cudaGraphDestroy(graph);
@@ -1535,18 +1648,18 @@ int Solver::cgsolve_padded(bool zero_guess, int ncgmax, double epscg, int *ierr,
       graph_kind = ifprec;
     }
     const long long per_graph = 2LL * U;
-    const long long nodes_per_iter = (ifprec == 2) ? 3 + sweep_launches() : 2;
+    const long long nodes = per_graph * ((ifprec == 2) ? 3 + sweep_launches() : 2) + (xg64 > 1 ? per_graph / xg64 : 0);
     long long launched = per_graph;
     int last_seen = -1, stalls = 0;
     CK(cudaGraphLaunch(graph_exec, stream));
-    launches += per_graph * nodes_per_iter;
+    launches += nodes;
     for (;;) {
       CK(cudaMemcpyAsync(h_state, d_state, sizeof(SolveState), cudaMemcpyDeviceToHost, stream));
       CK(cudaEventRecord(ev1, stream));
       if (launched < (long long)ncgmax + per_graph) {
         CK(cudaGraphLaunch(graph_exec, stream));
         launched += per_graph;
-        launches += per_graph * nodes_per_iter;
+        launches += nodes;
       }
       CK(cudaEventSynchronize(ev1));
       if (h_state->status != ST_RUNNING) break;
@@ -1701,7 +1814,7 @@ int Solver::getb_dev(const double *phi, double *br, double *bt, double *bp) {
 int Solver::energy_dev(const double *phi, double w[3]) {
   const int nb = 148 * 4;
   k_energy<<<nb, NTHR, 0, stream>>>(g, m, phi, d_partials);
-  k_energy_final<<<1, 32, 0, stream>>>(d_partials, nb, d_scalar);
+  k_energy_final<<<1, 96, 0, stream>>>(d_partials, nb, d_scalar);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(w, d_scalar, 3 * sizeof(double), cudaMemcpyDeviceToHost, stream));
   CK(cudaStreamSynchronize(stream));
@@ -1724,10 +1837,10 @@ float *Solver::r32_inner() { return ifprec == 2 ? dilu_r32(this) : m_r32; }
 int Solver::launch_iteration32(int u) {
   dim3 grid(g.nit, g.njt, g.nkc);
   dim3 gridu(g.nit, g.njt, g.nkc_u);
-  if (ifprec == 2) {  // the rotation of four directions: position u reads buffer u % 4, writes the next
-    p32_cur = m_p32q[u % X_GROUP];
-    p32_nxt = m_p32q[(u + 1) % X_GROUP];
-  }
+  // the rotation: position u reads buffer u % n, writes the next (the two buffers alternate without groups)
+  const int nrot = std::max(xg, 2);
+  p32_cur = m_p32q[u % nrot];
+  p32_nxt = m_p32q[(u + 1) % nrot];
   StencilArgs sa{};
   sa.p_new32 = p32_nxt;
   sa.q32 = m_q32;
@@ -1735,6 +1848,7 @@ int Solver::launch_iteration32(int u) {
   sa.s1p = d_s1p;
   sa.st = d_state;
   sa.partials = d_partials;
+  sa.xslot1 = xg > 1 ? 1 + u % xg : 0;
   UpdateArgs ua{};
   ua.x = d_x;
   ua.p32 = p32_nxt;
@@ -1751,23 +1865,21 @@ int Solver::launch_iteration32(int u) {
   if (ifprec == 2) {
     if ((stm = tensor_map(dilu_z32(this), false, &mp.m32[1]))) return stm;
     mp.m32[2] = mp.m32[0];
-    sa.xslot1 = 1 + u % X_GROUP;
     k_stencil<MODE_PCGZ32><<<grid, NTHR, StageLayout<MODE_PCGZ32>::smem, stream>>>(mp, g, m, sa);
-    // after every eighth iteration x += the eight iterations' alpha p (the
-    // direction of iteration slot i is buffer i + 1 mod 8); the sweeps with
-    // r32 -= alpha q, rho, beta and ernorm inside them; the south-ring sums of z
-    if (u % X_GROUP == X_GROUP - 1) {
-      XDirs dirs;
-      for (int i = 0; i < X_GROUP; i++) dirs.p[i] = m_p32q[(i + 1) % X_GROUP];
-      k_update_x_oct<<<xblocks, NTHR, 0, stream>>>(g, d_state, d_x, dirs);
-    }
-    int st = dilu_sweeps_fused(this, m_q32);
-    if (st) return st;
-    k_south_ring_z<<<dim3((g.nrm2 + 127) / 128, g.nkc_u), 128, 0, stream>>>(g, m, dilu_z32(this), d_s1z);
+    // after every eighth iteration x += the eight iterations' alpha p; the
+    // sweeps with r32 -= alpha q, rho, beta and ernorm inside them; the
+    // south-ring sums of z
+    int st;
+    if (u % xg == xg - 1 && (st = launch_x_group(m_p32q, nullptr, xg))) return st;
+    if ((st = dilu_sweeps_fused(this, m_q32))) return st;
+    k_south_ring_z<<<dim3((g.nrm2 + 127) / 128, g.nkc_u), 128, 0, stream>>>(g, m, (const float *)dilu_z32(this), d_s1z);
   } else {
     if ((stm = tensor_map(m_r32, false, &mp.m32[1])) || (stm = tensor_map(d_ai, false, &mp.m32[2]))) return stm;
-    k_stencil<MODE_PCG32><<<grid, NTHR, StageLayout<MODE_PCG32>::smem, stream>>>(mp, g, m, sa);
-    k_update<UPD_ITER, false, true><<<gridu, NTHR, 0, stream>>>(g, m, ua);
+    if (xg > 1) ua.x = nullptr;
+    CK(launch_pdl(k_stencil<MODE_PCG32>, grid, dim3(NTHR), StageLayout<MODE_PCG32>::smem, stream, mp, g, m, sa));
+    CK(launch_pdl(k_update<UPD_ITER, false, true>, gridu, dim3(NTHR), 0, stream, g, m, ua));
+    int st;
+    if (xg > 1 && u % xg == xg - 1 && (st = launch_x_group(m_p32q, nullptr, xg))) return st;
   }
   std::swap(p32_cur, p32_nxt);
   return pot3d_cuda_status(cudaGetLastError(), "launch_iteration32");
@@ -1890,14 +2002,13 @@ int Solver::mixed_solve(bool zero_guess, int ncgmax, double epscg, int *ierr, po
   const double est_iter_s = (ilu ? 100.0 : 60.0) * (double)g.Np / 5.0e12 + 6e-6;
   int U = (int)std::ceil(2.0e-3 / est_iter_s);
   U = std::max(1, std::min(U, 8));
-  if (ilu) U = (U + X_GROUP / 2 - 1) / (X_GROUP / 2) * (X_GROUP / 2);  // whole groups of eight iterations
-                                                                        // (the rotation and the x update)
+  U = (U + X_GROUP / 2 - 1) / (X_GROUP / 2) * (X_GROUP / 2);  // whole groups (the rotation and the x update)
   if (!graph32_exec || graph32_U != U) {
     if (graph32_exec) cudaGraphExecDestroy(graph32_exec);
     graph32_exec = nullptr;
     cudaGraph_t graph;
     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    for (int u = 0; u < 2 * U; u++) {  // even count (ILU(0): multiple of 8): the directions return to m_p32a
+    for (int u = 0; u < 2 * U; u++) {  // a multiple of 8: the directions return to m_p32a
       st = launch_iteration32(u);
       if (st) {
         cudaStreamEndCapture(stream, &graph);
@@ -1915,7 +2026,7 @@ int Solver::mixed_solve(bool zero_guess, int ncgmax, double epscg, int *ierr, po
   // kernels per iteration (ILU(0): stencil, sweeps, ring sums; plus one x
   // update per eight iterations)
   const long long nodes_per_iter = ilu ? 2 + sweep_launches() : 2;
-  const long long extra_per_graph = ilu ? 2LL * U / X_GROUP : 0;
+  const long long extra_per_graph = xg > 1 ? 2LL * U / xg : 0;
   double rho_ref = h_state->rho;  // r.z at the last FP64 residual
   int ncg_ref = 0;                // iterations at the last FP64 residual
   int n_refine = 0, stagnant = 0, stalls = 0;
@@ -1948,15 +2059,11 @@ int Solver::mixed_solve(bool zero_guess, int ncgmax, double epscg, int *ierr, po
     CK(cudaMemcpyAsync(h_state, d_state, sizeof(SolveState), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
     if (h_state->status != ST_RUNNING) break;
-    if (ilu && (ran % X_GROUP)) {
-      // the graph stopped inside a group of eight: the newest p is in buffer
-      // ran % 8, the next graph's first iteration reads buffer 0
-      CK(cudaMemcpyAsync(m_p32q[0], m_p32q[ran % X_GROUP], sizeof(float) * g.Np, cudaMemcpyDeviceToDevice,
-                         stream));
-    } else if (!ilu && (ran & 1)) {
-      // the graph stopped after an odd number of iterations: the newest p is
-      // in the buffer the next graph writes first
-      CK(cudaMemcpyAsync(p32_cur, p32_nxt, sizeof(float) * g.Np, cudaMemcpyDeviceToDevice, stream));
+    const int nrot = std::max(xg, 2);
+    if (ran % nrot) {
+      // the graph stopped inside the rotation: the newest p is in buffer
+      // ran % nrot, the next graph's first iteration reads buffer 0
+      CK(cudaMemcpyAsync(m_p32q[0], m_p32q[ran % nrot], sizeof(float) * g.Np, cudaMemcpyDeviceToDevice, stream));
     }
     // progress is judged over at least 10 iterations (updates that follow
     // each other closely near convergence neither count nor reset)
@@ -2458,6 +2565,7 @@ extern "C" int pot3d_gpu_batch_create_mode(int n, const pot3d_mesh_t *meshes, co
   for (int q = 0; q < n && !st; q++) {
     Solver *s = new Solver();
     B.inst.push_back(s);
+    s->batched = true;
     st = s->setup(&meshes[q], br0s[q], nullptr, pm_r1s[q], ifprec, precision);
     if (!st) {
       s->tk_default = s->g.tk;

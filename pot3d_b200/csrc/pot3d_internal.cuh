@@ -21,7 +21,8 @@ namespace pot3d {
 constexpr int TI = 64;      // radial points per tile (32 lanes x 2)
 constexpr int TJ = 8;       // theta rows per tile (one warp each)
 constexpr int NTHR = 256;   // threads per tile block
-constexpr int X_GROUP = 8;  // refined ILU(0) single solve: iterations per solution update
+constexpr int X_GROUP = 8;    // refined single solves: iterations per solution update
+constexpr int X_GROUP64 = 4;  // FP64 diagonal single solves
 constexpr int SROW = TI + 4;  // shared-memory row: [pad, halo-, 64 own, halo+, pad]
 
 // Mesh arrays on the device, 1-based Fortran indexing: arr[k] is Fortran
@@ -56,7 +57,7 @@ struct Geo {
 struct SolveState {
   double rho, rho_old, alpha, beta, bdotb, epsn, pq, epscg;
   double rho_true;  // refined mode: preconditioned FP64 residual norm^2
-  double xa[X_GROUP];  // refined ILU(0): alphas of the x updates applied in groups (0: none)
+  double xa[X_GROUP];  // alphas of the x updates applied in groups (0: none)
   int ncg, ncgmax, status, par;
   unsigned int cnt_a, cnt_b, cnt_c, pad0;
   int hist_cap, n_refine, inner, pad1;
@@ -153,6 +154,33 @@ __device__ bool last_block_sum(double part, double *partials, unsigned int *coun
                                double *total, double *sh) {
   const unsigned int b = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
   return last_block_sum_at<NT>(part, partials, counter, nblocks, b, total, sh);
+}
+
+// Programmatic dependent launch: the kernels of a diagonal-preconditioner
+// iteration are launched so that a kernel's blocks may start while the one
+// before drains, do what depends on the mesh alone, and wait here.  pdl_wait
+// returns once every earlier kernel has completed and its writes are visible;
+// without the launch attribute both are no-ops.  At 33x41x65, where an
+// iteration is two launches of 6 and 8 us, this takes 8% off it.  (The ILU(0)
+// iteration is launched plainly: with its persistent sweeps in the chain the
+// attribute cost 9% at 63x91x181.)
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                              const Args &...args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
 }  // namespace pot3d

@@ -42,13 +42,21 @@ struct Solver {
 
   // FP32-inner / FP64-refined mode (both preconditioners)
   float *m_p32a = nullptr, *m_p32b = nullptr, *m_r32 = nullptr, *m_q32 = nullptr;
-  // ILU(0): four directions in rotation (a, b and two more), so the solution
-  // update is applied once per four iterations
-  float *m_p32q[X_GROUP] = {};  // refined ILU(0): the directions of X_GROUP consecutive iterations
+  // The search directions of consecutive iterations rotate through xg
+  // buffers, so the solution update is applied once per xg iterations: xg =
+  // X_GROUP (refined) or X_GROUP64 (FP64, diagonal preconditioner), or 2 (the
+  // two buffers every solve has) where the others do not fit in memory; the
+  // FP64 ILU(0) solve updates x every iteration (xg 1).
+  float *m_p32q[X_GROUP] = {};
+  double *m_p64q[X_GROUP64] = {};
+  int xg = 1, xg64 = 1;
+  bool batched = false;  // a case of a batch (set before setup)
+  int x_buffers();   // allocate the rotation (setup)
+  int launch_x_group(const float *const *dirs32, const double *const *dirs64, int n);
   float *p32_cur = nullptr, *p32_nxt = nullptr;
   cudaGraphExec_t graph32_exec = nullptr;
   int graph32_U = 0;
-  int xblocks = 0;  // grid of the refined ILU(0) iterations' grouped solution update
+  int xblocks = 0;  // grid of the grouped solution update
   cudaEvent_t evm0 = nullptr, evm1 = nullptr;
   double refine_ratio = 1e-4;  // reliable update once the recurrence's r.z fell by this factor
   double stall_drop = 0.5;     // an update whose FP64 r.z fell by less than this factor is stagnant
@@ -82,7 +90,7 @@ struct Solver {
   int prec_padded(double *x);  // x <- M^-1 x
   int rhs_padded(double *b);
   int dot_padded(const double *x, const double *y, double *out_dev);
-  int launch_iteration();
+  int launch_iteration(int u);  // u: position in the captured graph
   // FP64 PCG on d_x (guess) / d_b (RHS).  d_r holds the residual on exit.
   int cgsolve_padded(bool zero_guess, int ncgmax, double epscg, int *ierr, pot3d_solve_info_t *info);
   int true_residual(double *out);  // ||b - A x|| / ||b|| of d_x, d_b
