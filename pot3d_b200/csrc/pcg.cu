@@ -143,9 +143,8 @@ __device__ __forceinline__ double apply_fac(const PtFac &f, double dpim, double 
 // fly, q = A p_new, p_new.q.  MODE_PCGZ: same with z read from an FP32
 // vector (the ILU(0) preconditioner's output).  MODE_PCG32 / MODE_PCGZ32:
 // the FP32-inner forms of PCG / PCGZ: p, r, z and q are stored in FP32 and
-// read as FP32 boxes, but p_new is formed and rounded once, and A p_new is
-// evaluated, in FP64 registers, so q is the FP64 product of the stored
-// FP32 p_new rounded once.  (An FP32 evaluation of a4*x - sum(a_nb*x_nb)
+// read as FP32 boxes; p_new is rounded once, and A p_new is evaluated in FP64
+// registers, so q is the FP64 product of the stored FP32 p_new rounded once.  (An FP32 evaluation of a4*x - sum(a_nb*x_nb)
 // cancels away the smooth modes that set the convergence of this
 // operator; FP64 arithmetic costs nothing here, the kernel is HBM-bound.)
 //
@@ -155,6 +154,12 @@ __device__ __forceinline__ double apply_fac(const PtFac &f, double dpim, double 
 //   j=1  ghost enters through a2 = -drh*dph*st(1)*dt_i(1) = 0 (st(1)=sin 0)
 //   j=nt ghost = 2*S1(i) - x(i,ntm1,k), S1 the ring mean of x at j=ntm1
 //   k    periodic wrap (seam_hhh, src/pot3d.F90:5746-5758)
+//
+// A thread marches along k with its own column's three planes in registers
+// and reads only the neighbours in e and j from shared memory, two columns per
+// access.  Measured against every neighbour read from the ring: PCGZ32 53.8 ->
+// 49.9 us at 127x181x361; whole solves, 127x181x361 FP32-refined diagonal 336
+// -> 302 ms and 121x181x361 FP64 diagonal 506 -> 455 ms.
 // ============================================================================
 enum { MODE_AX = 0, MODE_PCG = 1, MODE_PCGZ = 2, MODE_PCG32 = 3, MODE_PCGZ32 = 4 };
 
@@ -193,7 +198,7 @@ constexpr int TILE64_BYTES = BOX64_X * BOX_Y * 8;
 constexpr int TILE32_BYTES = BOX32_X * BOX_Y * 4;
 constexpr int TILE64_PITCH = (TILE64_BYTES + 127) / 128 * 128;
 constexpr int TILE32_PITCH = (TILE32_BYTES + 127) / 128 * 128;
-constexpr int PN_SLOTS = 4;
+constexpr int PN_SLOTS = 3;  // p_new planes in the ring: written, read, and still read by slower warps
 constexpr int MAX_TK = 512;  // k-planes per block at most (per-k factors in shared memory)
 constexpr uint32_t WAIT_LIMIT = 1u << 24;
 
@@ -225,7 +230,7 @@ struct StageLayout {
   static constexpr int bytes = n64 * TILE64_PITCH + n32 * TILE32_PITCH;
   static constexpr uint32_t tx = n64 * TILE64_BYTES + n32 * TILE32_BYTES;
   static constexpr int kfac_off = S_STAGES * bytes + PN_SLOTS * TILE64_BYTES + 128;
-  static constexpr int smem = kfac_off + 3 * 8 * MAX_TK;
+  static constexpr int smem = kfac_off + 4 * 8 * MAX_TK;
 };
 
 // Tensor maps of the stage inputs: m64[0] = x | p_old, m64[1] = r, m32 = a_i | z;
@@ -264,7 +269,7 @@ __device__ __forceinline__ void stencil_body(const StencilMaps &maps, const Geo 
   __shared__ double s1sh[TI];
   __shared__ int abort_flag;
 
-  double *kfac = reinterpret_cast<double *>(dyn + L::kfac_off);  // [tk][3]
+  double *kfac = reinterpret_cast<double *>(dyn + L::kfac_off);  // [tk][4]: dp_i(k-1), dp_i(k), dph(k)
   unsigned char *base = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~uintptr_t(127));
   // p_new ring [PN_SLOTS][BOX_Y][BOX64_X], FP64 in every mode: the FP32 modes
   // store each rounded p_new widened once, so the stencil reads it without
@@ -305,9 +310,9 @@ __device__ __forceinline__ void stencil_body(const StencilMaps &maps, const Geo 
     // dp_i(k-1), dp_i(k), dph(k) of the block's planes, staged once.
     for (int q = tid; q < k1 - k0; q += NTHR) {
       const int kf = k0 + q + 2;
-      kfac[3 * q + 0] = m.dp_i[kf - 1];
-      kfac[3 * q + 1] = m.dp_i[kf];
-      kfac[3 * q + 2] = m.dph[kf];
+      kfac[4 * q + 0] = m.dp_i[kf - 1];
+      kfac[4 * q + 1] = m.dp_i[kf];
+      kfac[4 * q + 2] = m.dph[kf];
     }
   };
   // The diagonal modes are launched before the kernel they follow has ended
@@ -335,9 +340,10 @@ __device__ __forceinline__ void stencil_body(const StencilMaps &maps, const Geo 
 
   const int p_first = k0 - 1;         // planes p_first .. k1 feed the stencil
   const int n_planes = k1 - k0 + 2;
+  int kk_issue = k0 == 0 ? g.npm2 - 1 : k0 - 1;  // plane of the next issue (periodic)
   auto issue = [&](int local) {       // thread 0: TMA loads of one plane
-    const int p = p_first + local;
-    const int kk = (p + g.npm2) % g.npm2;
+    const int kk = kk_issue;
+    kk_issue = kk + 1 == g.npm2 ? 0 : kk + 1;
     const int s = local % S_STAGES;
     unsigned char *st = base + s * L::bytes;
     mbar_expect_tx(&bar[s], L::tx);
@@ -371,66 +377,89 @@ __device__ __forceinline__ void stencil_body(const StencilMaps &maps, const Geo 
   const double pm = m.pm_r1;
   double dot = 0.0;
 
-  // p_new at (row, col) of the stage tile; col counts FP64 columns.  PCG32
-  // forms it in FP64 and rounds it once; PCGZ32 forms it with one FP32 fma
-  // (beta rounded to FP32 once per block): every operand is already FP32 and
-  // the result is stored in FP32, and the two conversions per operand and
-  // the rounding of an FP64 fma would load the conversion pipe, which bounds
-  // this kernel's issue, for a difference at the last bit of the FP32 value.
+  // p_new of two neighbouring columns (col even) or of one at (row, col) of
+  // the stage tile; col counts FP64 columns.  PCG32 forms p_new in FP64 and
+  // rounds it once: an FP32 pair (exact products, an exact sum) in its place is
+  // 2% faster but up to 30 times further off under cancellation, and 14% slower
+  // with a test of its rounding (302, 297 and 343 ms a solve at 127x181x361).
+  // PCGZ32 forms p_new with one FP32 fma (beta rounded to FP32 once per block):
+  // every operand is already FP32 and the result is stored in FP32.
   const float beta32 = (float)beta;
-  auto pnew_at = [&](const unsigned char *st, int row, int col) -> T {
-    const double *t0 = reinterpret_cast<const double *>(st);
-    if constexpr (MODE == MODE_PCG32) {
-      const float *f0 = reinterpret_cast<const float *>(st);
-      const float *f1 = reinterpret_cast<const float *>(st + TILE32_PITCH);
-      const float *f2 = reinterpret_cast<const float *>(st + 2 * TILE32_PITCH);
-      const int c = row * BOX32_X + col + 2;
-      return (float)fma(beta, (double)f0[c], (double)f2[c] * (double)f1[c]);
+  auto p64 = [&](float pv, float ai, float r) -> float {
+    return (float)fma(beta, (double)pv, (double)ai * (double)r);
+  };
+  auto pnew_at = [&](const unsigned char *st, int row, int col, auto pair) {
+    constexpr bool PAIR = decltype(pair)::value;
+    using D = typename std::conditional<PAIR, double2, double>::type;
+    using F = typename std::conditional<PAIR, float2, float>::type;
+    const int c64 = row * BOX64_X + col, c32 = row * BOX32_X + col + 2;
+    auto f32 = [&](int q) { return *reinterpret_cast<const F *>(reinterpret_cast<const float *>(st + q) + c32); };
+    auto f64 = [&](int q) { return *reinterpret_cast<const D *>(reinterpret_cast<const double *>(st + q) + c64); };
+    if constexpr (MODE == MODE_AX) {
+      return f64(0);
+    } else if constexpr (MODE == MODE_PCG32) {
+      const F pv = f32(0), r = f32(TILE32_PITCH), ai = f32(2 * TILE32_PITCH);
+      if constexpr (PAIR)
+        return make_float2(p64(pv.x, ai.x, r.x), p64(pv.y, ai.y, r.y));
+      else
+        return p64(pv, ai, r);
     } else if constexpr (MODE == MODE_PCGZ32) {
-      const float *f0 = reinterpret_cast<const float *>(st);
-      const float *f1 = reinterpret_cast<const float *>(st + TILE32_PITCH);
-      const int c = row * BOX32_X + col + 2;
-      return __fmaf_rn(beta32, f0[c], f1[c]);
-    } else if (MODE == MODE_AX) {
-      return t0[row * BOX64_X + col];
-    } else if (MODE == MODE_PCG) {
-      const double *t1 = reinterpret_cast<const double *>(st + TILE64_PITCH);
-      const float *t2 = reinterpret_cast<const float *>(st + 2 * TILE64_PITCH);
-      return fma(beta, t0[row * BOX64_X + col], (double)t2[row * BOX32_X + col + 2] * t1[row * BOX64_X + col]);
+      const F pv = f32(0), z = f32(TILE32_PITCH);
+      if constexpr (PAIR)
+        return make_float2(__fmaf_rn(beta32, pv.x, z.x), __fmaf_rn(beta32, pv.y, z.y));
+      else
+        return __fmaf_rn(beta32, pv, z);
+    } else if constexpr (MODE == MODE_PCG) {
+      const D pv = f64(0), r = f64(TILE64_PITCH);
+      const F ai = f32(2 * TILE64_PITCH);
+      if constexpr (PAIR)
+        return make_double2(fma(beta, pv.x, (double)ai.x * r.x), fma(beta, pv.y, (double)ai.y * r.y));
+      else
+        return fma(beta, pv, (double)ai * r);
     } else {
-      const float *t2 = reinterpret_cast<const float *>(st + TILE64_PITCH);
-      return fma(beta, t0[row * BOX64_X + col], (double)t2[row * BOX32_X + col + 2]);
+      const D pv = f64(0);
+      const F z = f32(TILE64_PITCH);
+      if constexpr (PAIR)
+        return make_double2(fma(beta, pv.x, (double)z.x), fma(beta, pv.y, (double)z.y));
+      else
+        return fma(beta, pv, (double)z);
     }
   };
 
+  // A thread's own column stays in registers (x at planes k-1, k, k+1); the
+  // ring serves the neighbours in e and j only.
   T2 own_cur{}, own_prev{};
+  double2 xm{}, xc{}, xn{};
+  const int own = (w + 1) * BOX64_X + 2 + el;
+  const bool first_e = e0 == 0, last_e0 = e0 == g.nrm2 - 1, last_e1 = e0 + 1 == g.nrm2 - 1;
+  long long id = g.idx(e0, jj, k0);
+  const long long id_step = (long long)g.NRP * g.ntm2;
+  double *slot = pn_ring;             // plane `local`
+  double *const ring_end = pn_ring + PN_SLOTS * (BOX_Y * BOX64_X);
   int local = 0;
   for (; local < n_planes; local++) {
     const int s = local % S_STAGES;
     const uint32_t parity = (local / S_STAGES) & 1;
     if (!mbar_wait(&bar[s], parity, WAIT_LIMIT)) abort_flag = 1;
     const unsigned char *st = base + s * L::bytes;
-    double *slot = pn_ring + (local % PN_SLOTS) * (BOX_Y * BOX64_X);
     // own pair (kept in registers in storage precision for the output of
     // this plane, which follows one plane later)
     own_prev = own_cur;
-    {
-      const int col = 2 + el;
-      own_cur.x = pnew_at(st, w + 1, col);
-      own_cur.y = pnew_at(st, w + 1, col + 1);
-      slot[(w + 1) * BOX64_X + col] = (double)own_cur.x;
-      slot[(w + 1) * BOX64_X + col + 1] = (double)own_cur.y;
-    }
+    own_cur = pnew_at(st, w + 1, 2 + el, std::true_type{});
+    xm = xc;
+    xc = xn;
+    xn = make_double2((double)own_cur.x, (double)own_cur.y);
+    *reinterpret_cast<double2 *>(slot + own) = xn;
     {  // halo: theta rows 0 and TJ+1 (128 points) and radial columns (16)
       if (tid < 2 * TI) {
         const int row = (tid < TI) ? 0 : TJ + 1;
         const int col = 2 + (tid & (TI - 1));
-        slot[row * BOX64_X + col] = (double)pnew_at(st, row, col);
+        slot[row * BOX64_X + col] = (double)pnew_at(st, row, col, std::false_type{});
       } else if (tid < 2 * TI + 2 * TJ) {
         const int q = tid - 2 * TI;
         const int row = 1 + (q >> 1);
         const int col = (q & 1) ? TI + 2 : 1;
-        slot[row * BOX64_X + col] = (double)pnew_at(st, row, col);
+        slot[row * BOX64_X + col] = (double)pnew_at(st, row, col, std::false_type{});
       }
     }
     __syncthreads();
@@ -439,53 +468,45 @@ __device__ __forceinline__ void stencil_body(const StencilMaps &maps, const Geo 
       issue(issued);
       issued++;
     }
-    if (local >= 2 && v0) {
-      const int kk = p_first + local - 1;  // plane whose stencil is now complete
-      const double *sc = pn_ring + ((local - 1) % PN_SLOTS) * (BOX_Y * BOX64_X);
-      const double *sm = pn_ring + ((local - 2) % PN_SLOTS) * (BOX_Y * BOX64_X);
-      const double *sp = slot;
-      const int kq = kk - k0;
-      const double dpim = kfac[3 * kq], dpip = kfac[3 * kq + 1], dphk = kfac[3 * kq + 2];
-      const int col = 2 + el;
-      const double *rowc = sc + (w + 1) * BOX64_X;
-      const double2 xc = *reinterpret_cast<const double2 *>(rowc + col);
-      const double2 xm = *reinterpret_cast<const double2 *>(sm + (w + 1) * BOX64_X + col);
-      const double2 xn = *reinterpret_cast<const double2 *>(sp + (w + 1) * BOX64_X + col);
-      const double2 xjm2 = *reinterpret_cast<const double2 *>(sc + w * BOX64_X + col);
-      const double2 xjp2 = *reinterpret_cast<const double2 *>(sc + (w + 2) * BOX64_X + col);
-      const double xim = (e0 == 0) ? xc.x : (double)rowc[col - 1];
-      const double xip = (e0 == g.nrm2 - 1) ? pm * xc.x : xc.y;
-      const double xjm = (jj == 0) ? 0.0 : xjm2.x;
-      const double xjp = south ? 2.0 * s1a - xc.x : xjp2.x;
-      const double y = apply_fac(f0, dpim, dpip, dphk, xm.x, xjm, xim, xc.x, xip, xjp, xn.x);
+    const double *sc = slot == pn_ring ? ring_end - BOX_Y * BOX64_X : slot - BOX_Y * BOX64_X;  // plane local - 1
+    slot = slot + BOX_Y * BOX64_X == ring_end ? pn_ring : slot + BOX_Y * BOX64_X;
+    if (local >= 2 && v0) {  // the stencil of plane kq = local - 2 of the chunk is complete
+      const double *kf = kfac + 4 * (local - 2);
+      const double2 dpi = *reinterpret_cast<const double2 *>(kf);
+      const double dpim = dpi.x, dpip = dpi.y, dphk = kf[2];
+      const double2 xjm2 = *reinterpret_cast<const double2 *>(sc + own - BOX64_X);
+      double2 xjp2 = *reinterpret_cast<const double2 *>(sc + own + BOX64_X);
+      const double xl = sc[own - 1], xr = sc[own + 2];
+      // j = 1: the coupling to the row below is an exact zero (st(1) = 0), and
+      // the row read there is zero
+      if (south) xjp2 = make_double2(2.0 * s1a - xc.x, 2.0 * s1b - xc.y);
+      const double xim = first_e ? xc.x : xl;
+      const double xip = last_e0 ? pm * xc.x : xc.y;
+      const double y = apply_fac(f0, dpim, dpip, dphk, xm.x, xjm2.x, xim, xc.x, xip, xjp2.x, xn.x);
       double y1 = 0.0;
       if (v1) {
-        const double xip1 = (e0 + 1 == g.nrm2 - 1) ? pm * xc.y : (double)rowc[col + 2];
-        const double xjm1 = (jj == 0) ? 0.0 : xjm2.y;
-        const double xjp1 = south ? 2.0 * s1b - xc.y : xjp2.y;
-        y1 = apply_fac(f1, dpim, dpip, dphk, xm.y, xjm1, xc.x, xc.y, xip1, xjp1, xn.y);
+        const double xip1 = last_e1 ? pm * xc.y : xr;
+        y1 = apply_fac(f1, dpim, dpip, dphk, xm.y, xjm2.y, xc.x, xc.y, xip1, xjp2.y, xn.y);
       }
-      const long long id = g.idx(e0, jj, kk);
       if constexpr (MODE == MODE_AX) {
         *reinterpret_cast<double2 *>(a.y + id) = make_double2(y, y1);
       } else if constexpr (F32) {
         // q is stored rounded; p.q uses the stored values, as the update does
-        // (own_prev is the stored p_new of this plane; the ring holds it
-        // exactly, so xc equals it)
+        // (own_prev is the stored p_new of this plane; xc holds it exactly)
         const float2 qv = make_float2((float)y, (float)y1);
-        const float2 own = make_float2(own_prev.x, v1 ? own_prev.y : 0.0f);
+        const float2 own2 = make_float2(own_prev.x, v1 ? own_prev.y : 0.0f);
         *reinterpret_cast<float2 *>(a.q32 + id) = qv;
-        *reinterpret_cast<float2 *>(a.p_new32 + id) = own;
+        *reinterpret_cast<float2 *>(a.p_new32 + id) = own2;
         dot = fma(xc.x, (double)qv.x, dot);
         dot = fma(v1 ? xc.y : 0.0, (double)qv.y, dot);
       } else {
-        double2 yv = make_double2(y, y1);
-        double2 own = make_double2(xc.x, v1 ? xc.y : 0.0);
-        *reinterpret_cast<double2 *>(a.q + id) = yv;
-        *reinterpret_cast<double2 *>(a.p_new + id) = own;
-        dot = fma(own.x, y, dot);
-        dot = fma(own.y, y1, dot);
+        const double2 own2 = make_double2(xc.x, v1 ? xc.y : 0.0);
+        *reinterpret_cast<double2 *>(a.q + id) = make_double2(y, y1);
+        *reinterpret_cast<double2 *>(a.p_new + id) = own2;
+        dot = fma(own2.x, y, dot);
+        dot = fma(own2.y, y1, dot);
       }
+      id += id_step;
     }
   }
 
@@ -1831,7 +1852,7 @@ float *Solver::r32_inner() { return ifprec == 2 ? dilu_r32(this) : m_r32; }
 // preconditioner: the PCG32 stencil (p = beta p + a_i r, q = A p, p.q ->
 // alpha) and the update (x += alpha p, r -= alpha q, r.(a_i r) -> rho,
 // beta, epsn).  ILU(0): the PCGZ32 stencil (p = z + beta p), at every
-// fourth u the solution update of the last four iterations, the fused
+// eighth u the solution update of the last eight iterations, the fused
 // sweeps (r32 -= alpha q; r32 -> z32; rho, beta, epsn), the south-ring sums
 // of z.
 int Solver::launch_iteration32(int u) {
