@@ -64,6 +64,25 @@ __global__ void __launch_bounds__(256) k_permute_rows(PermArgs a, long long rows
       perm_put(a, r * a.od[3] + c, inside && c < a.ie[3] ? ld(a.in, ib + c, a.in_dt) : 0.0f);
   }
 }
+// The same for FP32 rows stored as BF16 without accumulation (a layer's input
+// from its FP32 sums): eight columns a thread, two 16-byte loads and one
+// 16-byte store.  Rows, columns and strides that keep these aligned only
+// (pot3d_fno_permute); indexes are below 2^31.  47 -> 10.5 us for 32 of 64
+// columns at 359 x 719 positions.
+__global__ void __launch_bounds__(256) k_permute_rows8(PermArgs a, unsigned n) {
+  const unsigned cols = (unsigned)(a.od[3] / 8), n2 = (unsigned)a.od[2], n1 = (unsigned)a.od[1];
+  for (unsigned t = blockIdx.x * 256u + threadIdx.x; t < n; t += gridDim.x * 256u) {
+    const unsigned r = t / cols, c = (t - r * cols) * 8, o01 = r / n2, o2 = r - o01 * n2, o0 = o01 / n1, o1 = o01 - o0 * n1;
+    const bool inside = o0 < a.ie[0] && o1 < a.ie[1] && o2 < a.ie[2];
+    const float *in = reinterpret_cast<const float *>(a.in) + o0 * a.is[0] + o1 * a.is[1] + o2 * a.is[2] + c;
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 f = inside && c < a.ie[3] ? __ldg(reinterpret_cast<const float4 *>(in)) : z;
+    const float4 h = inside && c + 4 < a.ie[3] ? __ldg(reinterpret_cast<const float4 *>(in) + 1) : z;
+    __align__(16) __nv_bfloat162 o[4] = {__floats2bfloat162_rn(f.x, f.y), __floats2bfloat162_rn(f.z, f.w),
+                                         __floats2bfloat162_rn(h.x, h.y), __floats2bfloat162_rn(h.z, h.w)};
+    reinterpret_cast<uint4 *>(a.out)[t] = *reinterpret_cast<const uint4 *>(o);
+  }
+}
 // in's fastest axis is out axis q < 3: tiles of PT3 x 32 over (3, q) turned
 // in shared memory, so both sides move whole lines.  u, v: the other two out
 // axes.
@@ -116,33 +135,83 @@ __global__ void __launch_bounds__(256) k_permute_tile(const __grid_constant__ Ti
 }
 // One Fourier layer's sum and activation: pre[m][c] += spec[b][c][ph][th] for
 // m = (b, ph, th), and vout[m][0..63] (BF16) = act(pre[m][c]), zero for c >= W.
-// keep: pre's sum is stored (the backward pass needs it).  The spectral term
-// is turned in shared memory (32 theta points at once).
+// keep: pre's sum is stored (the backward pass needs it).  Bound by HBM and
+// L2 traffic (4 W + 2 W + 128 bytes a row), so the spectral term of 64 theta
+// points is turned in shared memory and a thread then forms eight channels of
+// one row: two 16-byte loads of pre and one 16-byte store (VEC: W a multiple of
+// four, pre and vout aligned; else one value at a time).  The W channels and the zeros beyond are
+// two loops, so that no lane of a warp idles through the activation.  33.7 ->
+// 25.1 us at 359 x 719 positions, W = 32, against one channel a lane.
+constexpr int SA_TH = 64;
+template <bool VEC>
 __global__ void __launch_bounds__(256) k_spec_act(float *__restrict__ pre, const __nv_bfloat16 *__restrict__ spec, int W,
                                                   int nph, int nth, int Pth, int act, int keep,
                                                   __nv_bfloat16 *__restrict__ vout) {
-  __shared__ float tile[64][33];
+  __shared__ float tile[64][SA_TH + 1];
   const int lane = threadIdx.x & 31, y = threadIdx.x >> 5;
-  const int tiles = (nth + 31) / 32, th0 = (int)(blockIdx.x % tiles) * 32;
+  const int tiles = (nth + SA_TH - 1) / SA_TH, th0 = (int)(blockIdx.x % tiles) * SA_TH;
   const int line = blockIdx.x / tiles, b = line / nph, ph = line % nph;
+  const int rows = min(SA_TH, nth - th0), nc = (W + 7) / 8;
+  const __nv_bfloat16 *sb = spec + ((long long)b * W * nph + ph) * Pth + th0;
+#pragma unroll 8
   for (int c = y; c < W; c += 8)
-    if (th0 + lane < nth)
-      tile[c][lane] = __bfloat162float(spec[(((long long)b * W + c) * nph + ph) * Pth + th0 + lane]);
+#pragma unroll
+    for (int t = lane; t < SA_TH; t += 32)
+      if (t < rows) tile[c][t] = __bfloat162float(sb[(long long)c * nph * Pth + t]);
   __syncthreads();
+  const long long m0 = (long long)line * nth + th0;
+  for (int i = threadIdx.x; i < rows * nc; i += 256) {
+    const int r = i / nc, c0 = (i - r * nc) * 8;
+    float *q = pre + (m0 + r) * W + c0;
+    float v[8];
 #pragma unroll
-  for (int r = y; r < 32; r += 8) {
-    const int th = th0 + r;
-    if (th >= nth) break;
-    const long long m = (long long)line * nth + th;
+    for (int k = 0; k < 8; k += 4) {
+      if (VEC) {
+        const float4 f = c0 + k < W ? *reinterpret_cast<const float4 *>(q + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[k] = f.x, v[k + 1] = f.y, v[k + 2] = f.z, v[k + 3] = f.w;
+      } else {
 #pragma unroll
-    for (int c = lane; c < 64; c += 32) {
-      float v = 0.0f;
-      if (c < W) {
-        v = pre[m * W + c] + tile[c][r];
-        if (keep) pre[m * W + c] = v;
-        if (act) v = gelu_f(v);
+        for (int h = k; h < k + 4; h++) v[h] = c0 + h < W ? q[h] : 0.0f;
       }
-      vout[m * 64 + c] = __float2bfloat16_rn(v);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (c0 + k < W) v[k] += tile[c0 + k][r];
+    if (keep) {
+#pragma unroll
+      for (int k = 0; k < 8; k += 4) {
+        if (VEC) {
+          if (c0 + k < W) *reinterpret_cast<float4 *>(q + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+        } else {
+#pragma unroll
+          for (int h = k; h < k + 4; h++)
+            if (c0 + h < W) q[h] = v[h];
+        }
+      }
+    }
+    __align__(16) __nv_bfloat162 o[4];
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      const float lo = act && c0 + k < W ? gelu_f(v[k]) : v[k], hi = act && c0 + k + 1 < W ? gelu_f(v[k + 1]) : v[k + 1];
+      o[k / 2] = __floats2bfloat162_rn(lo, hi);
+    }
+    __nv_bfloat16 *vo = vout + (m0 + r) * 64 + c0;
+    if (VEC) {
+      *reinterpret_cast<uint4 *>(vo) = *reinterpret_cast<const uint4 *>(o);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) vo[k] = o[k / 2].x, vo[k + 1] = o[k / 2].y;
+    }
+  }
+  const int nz = 8 - nc;
+  for (int i = threadIdx.x; i < rows * nz; i += 256) {
+    const int r = i / nz, c0 = (nc + i - r * nz) * 8;
+    __nv_bfloat16 *vo = vout + (m0 + r) * 64 + c0;
+    if (VEC) {
+      *reinterpret_cast<uint4 *>(vo) = make_uint4(0, 0, 0, 0);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; k++) vo[k] = __float2bfloat16_rn(0.0f);
     }
   }
 }
@@ -350,7 +419,12 @@ extern "C" int pot3d_fno_permute(const void *in, int in_dt, const long long *in_
   cudaStream_t s = (cudaStream_t)stream;
   if (q == 3) {
     const long long rows = od.d[0] * od.d[1] * od.d[2];
-    k_permute_rows<<<grid_for(rows * 32), 256, 0, s>>>(a, rows);
+    const long long n8 = rows * (a.od[3] / 8);
+    if (in_dt == DT_F32 && out_dt == DT_BF16 && !add && a.od[3] % 8 == 0 && a.ie[3] % 4 == 0 && a.is[0] % 4 == 0 &&
+        a.is[1] % 4 == 0 && a.is[2] % 4 == 0 && n8 < (1LL << 30) && ((uintptr_t)in | (uintptr_t)out) % 16 == 0)
+      k_permute_rows8<<<grid_for(n8), 256, 0, s>>>(a, (unsigned)n8);
+    else
+      k_permute_rows<<<grid_for(rows * 32), 256, 0, s>>>(a, rows);
   } else {
     const int u = q == 0 ? 1 : 0, v = q == 2 ? 1 : 2;
     const long long tq = (od.d[q] + 31) / 32, t3 = (od.d[3] + PT3 - 1) / PT3, nb = tq * t3 * od.d[u] * od.d[v];
@@ -377,12 +451,13 @@ extern "C" int pot3d_fno_permute(const void *in, int in_dt, const long long *in_
 
 extern "C" int pot3d_fno_spec_act(float *pre, const void *spec, int B, int W, int nph, int nth, int Pth, int act,
                                   int keep, void *vout, void *stream) {
-  const long long blocks = (long long)B * nph * ((nth + 31) / 32);
+  const long long blocks = (long long)B * nph * ((nth + SA_TH - 1) / SA_TH);
   if (B < 1 || W < 1 || W > 64 || nph < 1 || nth < 1 || Pth < nth || blocks > 0x7fffffff) {
     pot3d_set_error("pot3d_fno_spec_act: bad sizes");
     return POT3D_ERR_ARG;
   }
-  k_spec_act<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
+  const auto kernel = W % 4 == 0 && ((uintptr_t)pre | (uintptr_t)vout) % 16 == 0 ? k_spec_act<true> : k_spec_act<false>;
+  kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
       pre, reinterpret_cast<const __nv_bfloat16 *>(spec), W, nph, nth, Pth, act, keep,
       reinterpret_cast<__nv_bfloat16 *>(vout));
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_spec_act");
@@ -486,19 +561,34 @@ __global__ void __launch_bounds__(256) k_guess(const float *__restrict__ out, lo
 // levels, level i from source levels idx[i] and idx[i]+1 with weight w[i]
 // (outside [0, 1] at the ends: linear extrapolation).
 // A warp a position: the levels' indices and weights stay in L1.
+// Without the staging, which serves every row length, a row's values are
+// converted to FP64 twice for every output, and conversions issue at a tenth
+// of the FP32 rate; STAGED converts a row once into shared memory, a warp a row
+// (182 -> 150 us for 125 -> 253 levels at 359 x 719 positions; rows of up to 768
+// values, where eight fit 48 KB).
+template <bool STAGED>
 __global__ void __launch_bounds__(256) k_guess_resampled(const float *__restrict__ out, long long B, long long npos,
-                                                         int Rp, const int *__restrict__ idx,
+                                                         int Rp, int Rs, const int *__restrict__ idx,
                                                          const double *__restrict__ w, int R,
                                                          const double *__restrict__ sigma, double *__restrict__ x) {
+  extern __shared__ double row_s[];
   const int lane = threadIdx.x & 31;
+  double *row = row_s + (threadIdx.x >> 5) * Rs;
   for (long long bp = blockIdx.x * 8LL + (threadIdx.x >> 5); bp < B * npos; bp += gridDim.x * 8LL) {
     const double sg = sigma[bp / npos];
+    const float *o = out + bp * Rp;
+    if (STAGED) {
+#pragma unroll 4
+      for (int i = lane; i < Rs; i += 32) row[i] = (double)o[i];
+      __syncwarp();
+    }
 #pragma unroll 4
     for (int i = lane; i < R; i += 32) {
-      const float *o = out + bp * Rp + idx[i];
-      const double lo = (double)o[0], hi = (double)o[1];
+      const int q = idx[i];
+      const double lo = STAGED ? row[q] : (double)o[q], hi = STAGED ? row[q + 1] : (double)o[q + 1];
       x[bp * R + i] = fma(w[i], hi - lo, lo) * sg;
     }
+    if (STAGED) __syncwarp();
   }
 }
 }  // namespace
@@ -510,8 +600,12 @@ extern "C" int pot3d_fno_guess_resampled(const float *out, long long B, long lon
     pot3d_set_error("pot3d_fno_guess_resampled: bad sizes");
     return POT3D_ERR_ARG;
   }
-  k_guess_resampled<<<grid_for(B * npos * 32), 256, 0, (cudaStream_t)stream>>>(out, B, npos, Rp, idx, w, R, sigma,
-                                                                              x);
+  const unsigned blocks = grid_for(B * npos * 32);
+  const size_t smem = 8 * sizeof(double) * (size_t)Rs;  // a row for each of the eight warps
+  if (smem <= 48 * 1024)
+    k_guess_resampled<true><<<blocks, 256, smem, (cudaStream_t)stream>>>(out, B, npos, Rp, Rs, idx, w, R, sigma, x);
+  else
+    k_guess_resampled<false><<<blocks, 256, 0, (cudaStream_t)stream>>>(out, B, npos, Rp, Rs, idx, w, R, sigma, x);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_guess_resampled");
 }
 

@@ -112,3 +112,37 @@ def test_relmse_and_colsum(cuda, b, npos, R, ldp):
     s = colsum(flat, R, ldp, new((R,), "f32"))
     ref = flat[:, :R].double().sum(0)
     assert bool(((s.double() - ref).abs() <= 4 * EPS32 * np.sqrt(b * npos) * flat[:, :R].double().abs().sum(0) + 1e-30).all())
+
+
+@pytest.mark.parametrize("rows,cols,out_cols", [(1, 4, 8), (1001, 32, 64), (37, 128, 128), (5, 64, 32), (9, 12, 40)])
+def test_permute_rows_eight_columns_a_thread(cuda, rows, cols, out_cols):
+    import torch
+    from pot3d_b200.fno import permute
+    x = _t((2, 3, rows, cols), cuda, 11)
+    ref = torch.nn.functional.pad(x[..., :out_cols], (0, max(0, out_cols - cols))).bfloat16()
+    shifted = torch.empty(2 * 3 * rows * cols + 1, device=cuda)[1:].view(x.shape).copy_(x)  # not 16-byte aligned
+    for src in (x, shifted):
+        out = torch.full((2, 3, rows, out_cols), 7.0, device=cuda, dtype=torch.bfloat16)
+        assert torch.equal(permute(src, x.shape, out, out.shape, (0, 1, 2, 3)), ref)
+    out = torch.full((3, 2, rows, out_cols), 7.0, device=cuda, dtype=torch.bfloat16)
+    assert torch.equal(permute(x, x.shape, out, out.shape, (1, 0, 2, 3)), ref.transpose(0, 1))
+
+
+@pytest.mark.parametrize("b,npos,rs,r", [(1, 1, 2, 1), (2, 1201, 125, 253), (1, 9, 768, 800), (1, 9, 769, 31)])
+def test_guess_resampled(cuda, b, npos, rs, r):
+    import torch
+    from pot3d_b200 import _lib
+    from pot3d_b200.fno import _L
+    rp = (rs + 63) // 64 * 64
+    out = _t((b, npos, rp), cuda, 12)
+    idx = torch.randint(0, rs - 1, (r,), device=cuda, dtype=torch.int32, generator=torch.Generator(cuda).manual_seed(13))
+    w, sigma = 1.2 * _t((r,), cuda, 14, torch.float64), _t((b,), cuda, 15, torch.float64)
+    x = torch.empty((b, npos, r), device=cuda, dtype=torch.float64)
+    _lib.check(_L().pot3d_fno_guess_resampled(*[C.c_void_p(out.data_ptr()), b, npos, rp, rs], C.c_void_p(idx.data_ptr()),
+                                              C.c_void_p(w.data_ptr()), r, C.c_void_p(sigma.data_ptr()),
+                                              C.c_void_p(x.data_ptr()), None))
+    torch.cuda.synchronize()
+    lo, hi = out.double()[..., idx.long()], out.double()[..., idx.long() + 1]
+    # the same operations but for the fma's missing rounding: two roundings of the terms' magnitudes and the product's
+    tol = 4 * 2.0 ** -53 * (lo.abs() + (w * (hi - lo)).abs()) * sigma.abs().view(-1, 1, 1)
+    assert bool(((x - (lo + w * (hi - lo)) * sigma.view(-1, 1, 1)).abs() <= tol).all())
