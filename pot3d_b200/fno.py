@@ -30,13 +30,13 @@ from dataclasses import dataclass
 import numpy as np
 
 from . import _lib
-from .tc import tc_gemm
+from .tc import LAUNCHES, raw_stream, tc_gemm
 
 F32, BF16 = 0, 1
+_Dims, _Perm = C.c_longlong * 4, C.c_int * 4
 
 
 def _count():
-    from .tc import LAUNCHES
     LAUNCHES[0] += 1
 
 
@@ -64,7 +64,7 @@ def _L():
 
 def _stream():
     import torch
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(raw_stream(torch.cuda.current_device()))
 
 
 def _dt(t):
@@ -74,12 +74,9 @@ def _dt(t):
 
 def permute(inp, in_dims, out, out_dims, perm, add=False):
     """out[o] = inp[i] with i[perm[a]] = o[a]; zero outside inp (pad/crop)."""
-    idd = (C.c_longlong * 4)(*in_dims)
-    odd = (C.c_longlong * 4)(*out_dims)
-    pp = (C.c_int * 4)(*perm)
     _count()
-    _lib.check(_L().pot3d_fno_permute(C.c_void_p(inp.data_ptr()), _dt(inp), idd, C.c_void_p(out.data_ptr()),
-                                      _dt(out), odd, pp, 1 if add else 0, _stream()))
+    _lib.check(_L().pot3d_fno_permute(inp.data_ptr(), _dt(inp), _Dims(*in_dims), out.data_ptr(), _dt(out),
+                                      _Dims(*out_dims), _Perm(*perm), 1 if add else 0, _stream()))
     return out
 
 
