@@ -4,12 +4,13 @@
 // the boundary trick, phi finalisation, getb + magnetic energy).
 //
 // Per PCG iteration (classical PCG of cgsolve, src/pot3d.F90:4336-4365)
-// exactly two kernels run, both tiled over (i, j, k) with TIxTJ tiles that
-// march along k:
+// two kernels run, both tiled over (i, j, k) with TIxTJ tiles that march
+// along k:
 //   k_stencil<PCG> : p = beta*p + z (z = a_i*r formed on the fly),
 //                    q = A p, and the p.q partial sums -> alpha
 //   k_update<>     : x += alpha p, r -= alpha q, z = a_i*r, r.z -> rho,
-//                    beta, epsn (ernorm, src/pot3d.F90:4430-4433)
+//                    beta, epsn (ernorm, src/pot3d.F90:4430-4433); on grids
+//                    above L2 x is left to k_update_x_group, once a group
 // All scalars stay on the device (SolveState); the host only polls the
 // convergence flag between CUDA-graph launches of several iterations.
 #include <cuda_runtime.h>
