@@ -233,27 +233,46 @@ __global__ void __launch_bounds__(256) k_gelu(const float *__restrict__ pre, lon
     }
 }
 
-// out[c] = sum_m in[m][c], c < C: per-block partial sums in a fixed order.  A
-// block sums 32 columns (a lane a column, so a warp reads a line of a row).
-constexpr int CS_ROWS = 32;  // rows a block reads at once
+// out[c] = sum_m in[m][c], c < C: partial sums in a fixed order, 64 blocks of
+// 256 chains of rows (chain t of block b takes rows 256 b + t, then every
+// 256 * 64th) and a binary tree over a block's chains.  A block sums 32
+// columns (a lane a column, so a warp reads a line of a row), a warp eight
+// chains of each; the tree's three widest levels are a thread's own chains.
+constexpr int CS_ROWS = 32;      // chains a block reads at once
+constexpr int CS_CHAINS = 256;   // chains of a block
 __global__ void __launch_bounds__(32 * CS_ROWS) k_colsum(const float *__restrict__ in, long long M, int C, int ld,
                                                          float *__restrict__ part) {
+  constexpr int NC = CS_CHAINS / CS_ROWS;
   const int lane = threadIdx.x & 31, y = threadIdx.x >> 5, c = blockIdx.y * 32 + lane;
-  float s = 0.0f;
+  float s[NC] = {};
   if (c < C) {
-#pragma unroll 8
-    for (long long m = blockIdx.x * (long long)CS_ROWS + y; m < M; m += gridDim.x * (long long)CS_ROWS)
-      s += in[m * ld + c];
-  }
-  __shared__ float red[CS_ROWS][32];
-  red[y][lane] = s;
-  __syncthreads();
-  if (y == 0 && c < C) {
-    float t = 0.0f;
+    const float *p = in + c;
+    const long long step = gridDim.x * (long long)CS_CHAINS;
+    long long m0 = blockIdx.x * (long long)CS_CHAINS + y;
+#pragma unroll 2
+    for (; m0 + CS_ROWS * (NC - 1) < M; m0 += step) {
+      float v[NC];
 #pragma unroll
-    for (int q = 0; q < CS_ROWS; q++) t += red[q][lane];
-    part[(long long)c * gridDim.x + blockIdx.x] = t;
+      for (int j = 0; j < NC; j++) v[j] = p[(m0 + CS_ROWS * j) * ld];
+#pragma unroll
+      for (int j = 0; j < NC; j++) s[j] += v[j];
+    }
+#pragma unroll
+    for (int j = 0; j < NC; j++)
+      if (m0 + CS_ROWS * j < M) s[j] += p[(m0 + CS_ROWS * j) * ld];
   }
+#pragma unroll
+  for (int o = NC / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int j = 0; j < o; j++) s[j] += s[j + o];
+  __shared__ float red[CS_ROWS][32];
+  red[y][lane] = s[0];
+  __syncthreads();
+  for (int o = CS_ROWS / 2; o > 0; o >>= 1) {
+    if (y < o) red[y][lane] += red[y + o][lane];
+    __syncthreads();
+  }
+  if (y == 0 && c < C) part[(long long)c * gridDim.x + blockIdx.x] = red[0][lane];
 }
 __global__ void k_colsum_final(const float *__restrict__ part, int nb, int C, float *__restrict__ out, int add) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;

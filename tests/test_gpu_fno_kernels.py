@@ -114,6 +114,29 @@ def test_relmse_and_colsum(cuda, b, npos, R, ldp):
     assert bool(((s.double() - ref).abs() <= 4 * EPS32 * np.sqrt(b * npos) * flat[:, :R].double().abs().sum(0) + 1e-30).all())
 
 
+@pytest.mark.parametrize("m,c,ld", [(1, 1, 1), (255, 33, 40), (257, 32, 32), (16384 + 31, 125, 128), (5 * 16384 + 300, 7, 64)])
+def test_colsum_order(cuda, m, c, ld):
+    """Bit for bit the stated order: 64 blocks of 256 chains of rows, a binary
+    tree over a block's chains, then the blocks one after the other."""
+    import torch
+    from pot3d_b200.fno import colsum, new
+    x = _t((m, ld), cuda, 16)
+    steps = -(-m // (64 * 256))
+    rows = torch.zeros((steps * 64 * 256, c), device=cuda)
+    rows[:m] = x[:, :c]
+    rows = rows.view(steps, 64, 256, c)
+    s = torch.zeros((64, 256, c), device=cuda)
+    for k in range(steps):
+        s = s + rows[k]
+    while s.shape[1] > 1:
+        h = s.shape[1] // 2
+        s = s[:, :h] + s[:, h:]
+    ref = torch.zeros(c, device=cuda)
+    for b in range(64):
+        ref = ref + s[b, 0]
+    assert torch.equal(colsum(x, c, ld, new((c,), "f32")), ref)
+
+
 @pytest.mark.parametrize("rows,cols,out_cols", [(1, 4, 8), (1001, 32, 64), (37, 128, 128), (5, 64, 32), (9, 12, 40)])
 def test_permute_rows_eight_columns_a_thread(cuda, rows, cols, out_cols):
     import torch
