@@ -602,19 +602,21 @@ __device__ __forceinline__ void update_body(const Geo &g, const DevMesh &m, cons
 #pragma unroll 4
     for (int kk = k0; kk < k1; kk++) {
       const long long id = g.idx(e0, jj, kk);
+      // q, p and z come from the kernels before: ordinary loads (see pdl_wait),
+      // q's ahead of x's store
       double2 rv = R32 ? widen2(*reinterpret_cast<const float2 *>(a.r32 + id))
                        : *reinterpret_cast<const double2 *>(a.r + id);
       if (KIND == UPD_ITER) {
+        const double2 qv = R32 ? widen2(*reinterpret_cast<const float2 *>(a.q32 + id))
+                               : *reinterpret_cast<const double2 *>(a.q + id);
         if (a.x) {  // else applied in groups of iterations (k_update_x_group)
           double2 xv = *reinterpret_cast<const double2 *>(a.x + id);
-          const double2 pv = R32 ? widen2(__ldg(reinterpret_cast<const float2 *>(a.p32 + id)))
-                                 : __ldg(reinterpret_cast<const double2 *>(a.p + id));
+          const double2 pv = R32 ? widen2(*reinterpret_cast<const float2 *>(a.p32 + id))
+                                 : *reinterpret_cast<const double2 *>(a.p + id);
           xv.x = fma(alpha, pv.x, xv.x);
           xv.y = fma(alpha, pv.y, xv.y);
           *reinterpret_cast<double2 *>(a.x + id) = xv;
         }
-        const double2 qv = R32 ? widen2(__ldg(reinterpret_cast<const float2 *>(a.q32 + id)))
-                               : __ldg(reinterpret_cast<const double2 *>(a.q + id));
         rv.x = fma(-alpha, qv.x, rv.x);
         rv.y = fma(-alpha, qv.y, rv.y);
         if (R32) {
@@ -628,7 +630,7 @@ __device__ __forceinline__ void update_body(const Geo &g, const DevMesh &m, cons
       if (!v1) rv.y = 0.0;
       double zx, zy;
       if (ZIN) {
-        const float2 zv = __ldg(reinterpret_cast<const float2 *>(a.z32 + id));
+        const float2 zv = *reinterpret_cast<const float2 *>(a.z32 + id);
         zx = zv.x;
         zy = zv.y;
       } else {
@@ -666,8 +668,10 @@ __device__ __forceinline__ void update_body(const Geo &g, const DevMesh &m, cons
   }
 }
 
+// Six blocks an SM (40 registers), four of the batched form: without the bound
+// the ordinary loads of four planes are hoisted into 54 registers.
 template <int KIND, bool ZIN, bool R32 = false>
-__global__ void __launch_bounds__(NTHR) k_update(Geo g, DevMesh m, UpdateArgs a) {
+__global__ void __launch_bounds__(NTHR, 6) k_update(Geo g, DevMesh m, UpdateArgs a) {
   update_body<KIND, ZIN, R32>(g, m, a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -787,12 +791,12 @@ __global__ void __launch_bounds__(NTHR) k_update_x_group(Geo g, const SolveState
 #pragma unroll
     for (int i = 0; i < G; i++) {
       if constexpr (sizeof(T) == 4) {
-        const float4 v = __ldg(reinterpret_cast<const float4 *>(d.p[i] + id));
+        const float4 v = *reinterpret_cast<const float4 *>(d.p[i] + id);
         v0[i] = make_double2((double)v.x, (double)v.y);
         v1[i] = make_double2((double)v.z, (double)v.w);
       } else {
-        v0[i] = __ldg(reinterpret_cast<const double2 *>(d.p[i] + id));
-        v1[i] = __ldg(reinterpret_cast<const double2 *>(d.p[i] + id + 2));
+        v0[i] = *reinterpret_cast<const double2 *>(d.p[i] + id);
+        v1[i] = *reinterpret_cast<const double2 *>(d.p[i] + id + 2);
       }
     }
 #pragma unroll
@@ -2199,7 +2203,7 @@ __global__ void __launch_bounds__(NTHR, MODE == MODE_PCGZ32 ? 3 : 2) k_stencil_b
 // UPD_ITER with the diagonal preconditioner, UPD_ZDOT after the ILU(0) sweeps
 // (R32: the FP32-inner forms).
 template <int KIND, bool ZIN, bool R32 = false>
-__global__ void __launch_bounds__(NTHR) k_update_batch(const BatchInst *__restrict__ in, int n, int par) {
+__global__ void __launch_bounds__(NTHR, 4) k_update_batch(const BatchInst *__restrict__ in, int n, int par) {
   const int i = batch_find(in, n, blockIdx.x, BATCH_UPDATE);
   const BatchInst &I = in[i];
   const Geo &g = I.g;

@@ -159,8 +159,11 @@ __device__ bool last_block_sum(double part, double *partials, unsigned int *coun
 // Programmatic dependent launch: the kernels of a diagonal-preconditioner
 // iteration are launched so that a kernel's blocks may start while the one
 // before drains, do what depends on the mesh alone, and wait here.  pdl_wait
-// returns once every earlier kernel has completed and its writes are visible;
-// without the launch attribute both are no-ops.  At 33x41x65, where an
+// returns once every earlier kernel has completed and its writes are visible
+// to ordinary loads and TMA; without the launch attribute both are no-ops.
+// Such a kernel is resident while its predecessor still writes, so nothing
+// that any iteration's kernel writes is read-only for its lifetime: __ldg and
+// const __restrict__ are for what setup wrote (the mesh, a_i).  At 33x41x65, where an
 // iteration is two launches of 6 and 8 us, this takes 8% off it.  (The ILU(0)
 // iteration is launched plainly: with its persistent sweeps in the chain the
 // attribute cost 9% at 63x91x181.)
