@@ -15,7 +15,8 @@
  *    cgsolve (src/pot3d.F90:4231-4369) and the pieces of potfld around it
  *    (RHS, phi finalisation, energies).  They return a status code
  *    (POT3D_OK = 0) and never exit; pot3d_gpu_last_error() describes the
- *    most recent failure on the calling thread.
+ *    most recent failure on the calling thread.  Calls on one handle from
+ *    several threads take turns.
  *
  * Layout conventions follow the reference exactly:
  *  - 1-D mesh arrays are the local_mesh arrays of one rank (Fortran element
@@ -216,6 +217,13 @@ int pot3d_gpu_time_kernels(pot3d_gpu_solver *s, int reps, double ms[2], double b
  * refined mode.  No counterpart in the reference (its timers cover whole
  * preconditioner calls, src/pot3d.F90 timing.out "PC"). */
 int pot3d_gpu_time_sweeps(pot3d_gpu_solver *s, int reps, double ms[2]);
+
+/* Iterations per update of the solution in this handle's solves: 1, or the
+ * length of the group that is applied at once (4 for FP64 with the diagonal
+ * preconditioner and 8 for the refined mode with it, where an iteration's
+ * vectors outgrow the device's L2 cache; 8 for refined ILU(0)).  The solution
+ * is the same bits either way.  0 for a null handle. */
+int pot3d_gpu_update_group(const pot3d_gpu_solver *s);
 
 /* Failure-detection check of the ILU(0) wavefront sweeps (ifprec = 2): runs
  * the forward sweep with one tile left undone, so the waits of the tiles

@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <mutex>
 #include <new>
 
 #include "pot3d_internal.cuh"
@@ -9,10 +10,11 @@
 
 using pot3d::Solver;
 
+// Calls on one handle take turns: they share the solver's scratch vectors,
+// and a solve's search directions pass through them.
 struct pot3d_gpu_solver {
   Solver s;
-  double *d_io = nullptr;  // device staging buffer, reference packed layout (N)
-  double *d_io2 = nullptr;
+  std::mutex turn;
 };
 
 #define CKS(call)                                                 \
@@ -43,8 +45,6 @@ extern "C" int pot3d_gpu_create(const pot3d_mesh_t *mesh, const double *br0, con
     return POT3D_ERR_NOMEM;
   }
   int st = h->s.setup(mesh, br0, br1, pm_r1, ifprec, precision);
-  if (st == POT3D_OK) st = h->s.alloc((void **)&h->d_io, sizeof(double) * (size_t)h->s.g.N);
-  if (st == POT3D_OK) st = h->s.alloc((void **)&h->d_io2, sizeof(double) * (size_t)h->s.g.N);
   if (st != POT3D_OK) {
     delete h;
     return st;
@@ -63,10 +63,11 @@ extern "C" long pot3d_gpu_size(const pot3d_gpu_solver *h) { return h ? (long)h->
 extern "C" int pot3d_gpu_rhs(pot3d_gpu_solver *h, double *rhs) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   Solver &s = h->s;
   if ((st = s.rhs_padded(s.d_tmp))) return st;
-  if ((st = s.unpack(s.d_tmp, h->d_io))) return st;
-  CKS(cudaMemcpyAsync(rhs, h->d_io, sizeof(double) * s.g.N, cudaMemcpyDeviceToHost, s.stream));
+  if ((st = s.unpack(s.d_tmp, s.d_io))) return st;
+  CKS(cudaMemcpyAsync(rhs, s.d_io, sizeof(double) * s.g.N, cudaMemcpyDeviceToHost, s.stream));
   CKS(cudaStreamSynchronize(s.stream));
   return POT3D_OK;
 }
@@ -112,6 +113,7 @@ extern "C" int pot3d_gpu_cgsolve_dev(pot3d_gpu_solver *h, double *x, double *r, 
                                      int *ierr, pot3d_solve_info_t *info) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   return solve_common(h, x, r, N, ncgmax, epscg, ierr, info, x, r);
 }
 
@@ -119,17 +121,18 @@ extern "C" int pot3d_gpu_cgsolve(pot3d_gpu_solver *h, double *x, double *r, long
                                  int *ierr, pot3d_solve_info_t *info) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   Solver &s = h->s;
   if (N != (long)s.g.N) {
     pot3d_set_error("cgsolve: N does not match the mesh");
     return POT3D_ERR_ARG;
   }
   const size_t b = sizeof(double) * (size_t)N;
-  CKS(cudaMemcpyAsync(h->d_io, x, b, cudaMemcpyHostToDevice, s.stream));
-  CKS(cudaMemcpyAsync(h->d_io2, r, b, cudaMemcpyHostToDevice, s.stream));
-  if ((st = solve_common(h, h->d_io, h->d_io2, N, ncgmax, epscg, ierr, info, h->d_io, h->d_io2))) return st;
-  CKS(cudaMemcpyAsync(x, h->d_io, b, cudaMemcpyDeviceToHost, s.stream));
-  CKS(cudaMemcpyAsync(r, h->d_io2, b, cudaMemcpyDeviceToHost, s.stream));
+  CKS(cudaMemcpyAsync(s.d_io, x, b, cudaMemcpyHostToDevice, s.stream));
+  CKS(cudaMemcpyAsync(s.d_io2, r, b, cudaMemcpyHostToDevice, s.stream));
+  if ((st = solve_common(h, s.d_io, s.d_io2, N, ncgmax, epscg, ierr, info, s.d_io, s.d_io2))) return st;
+  CKS(cudaMemcpyAsync(x, s.d_io, b, cudaMemcpyDeviceToHost, s.stream));
+  CKS(cudaMemcpyAsync(r, s.d_io2, b, cudaMemcpyDeviceToHost, s.stream));
   CKS(cudaStreamSynchronize(s.stream));
   return POT3D_OK;
 }
@@ -147,11 +150,12 @@ extern "C" int pot3d_gpu_history(const pot3d_gpu_solver *h, double *eps, int cap
 extern "C" int pot3d_gpu_finalize_phi(pot3d_gpu_solver *h, const double *x, double *phi) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   Solver &s = h->s;
   const size_t nphi = (size_t)s.g.nr * s.g.nt * s.g.np;
   if (!s.d_phi && (st = s.alloc((void **)&s.d_phi, sizeof(double) * nphi))) return st;
-  CKS(cudaMemcpyAsync(h->d_io, x, sizeof(double) * s.g.N, cudaMemcpyHostToDevice, s.stream));
-  if ((st = s.pack(h->d_io, s.d_tmp))) return st;
+  CKS(cudaMemcpyAsync(s.d_io, x, sizeof(double) * s.g.N, cudaMemcpyHostToDevice, s.stream));
+  if ((st = s.pack(s.d_io, s.d_tmp))) return st;
   if ((st = s.finalize_phi_dev(s.d_tmp, s.d_phi))) return st;
   CKS(cudaMemcpyAsync(phi, s.d_phi, sizeof(double) * nphi, cudaMemcpyDeviceToHost, s.stream));
   CKS(cudaStreamSynchronize(s.stream));
@@ -161,6 +165,7 @@ extern "C" int pot3d_gpu_finalize_phi(pot3d_gpu_solver *h, const double *x, doub
 extern "C" int pot3d_gpu_energy(pot3d_gpu_solver *h, const double *phi, double w[3]) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   Solver &s = h->s;
   const size_t nphi = (size_t)s.g.nr * s.g.nt * s.g.np;
   if (!s.d_phi && (st = s.alloc((void **)&s.d_phi, sizeof(double) * nphi))) return st;
@@ -172,6 +177,7 @@ extern "C" int pot3d_gpu_fields(pot3d_gpu_solver *h, const double *x, double *ph
                                 double *bp, double w[3]) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   if (!x) {
     pot3d_set_error("pot3d_gpu_fields: null x");
     return POT3D_ERR_ARG;
@@ -180,8 +186,8 @@ extern "C" int pot3d_gpu_fields(pot3d_gpu_solver *h, const double *x, double *ph
   const size_t nr = s.g.nr, nt = s.g.nt, np = s.g.np;
   const size_t nphi = nr * nt * np;
   if (!s.d_phi && (st = s.alloc((void **)&s.d_phi, sizeof(double) * nphi))) return st;
-  CKS(cudaMemcpyAsync(h->d_io, x, sizeof(double) * s.g.N, cudaMemcpyHostToDevice, s.stream));
-  if ((st = s.pack(h->d_io, s.d_tmp))) return st;
+  CKS(cudaMemcpyAsync(s.d_io, x, sizeof(double) * s.g.N, cudaMemcpyHostToDevice, s.stream));
+  if ((st = s.pack(s.d_io, s.d_tmp))) return st;
   if ((st = s.finalize_phi_dev(s.d_tmp, s.d_phi))) return st;
   if (phi) CKS(cudaMemcpyAsync(phi, s.d_phi, sizeof(double) * nphi, cudaMemcpyDeviceToHost, s.stream));
   if (br || bt || bp) {
@@ -215,6 +221,7 @@ extern "C" int pot3d_gpu_fields(pot3d_gpu_solver *h, const double *x, double *ph
 extern "C" int pot3d_gpu_ax_dev(pot3d_gpu_solver *h, const double *x, double *y) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   Solver &s = h->s;
   if ((st = s.pack(x, s.d_tmp))) return st;
   if ((st = s.ax_padded(s.d_tmp, s.d_q))) return st;
@@ -226,6 +233,7 @@ extern "C" int pot3d_gpu_ax_dev(pot3d_gpu_solver *h, const double *x, double *y)
 extern "C" int pot3d_gpu_prec_dev(pot3d_gpu_solver *h, double *x) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   Solver &s = h->s;
   if ((st = s.pack(x, s.d_tmp))) return st;
   if ((st = s.prec_padded(s.d_tmp))) return st;
@@ -247,9 +255,10 @@ __global__ static void k_unpack_f(pot3d::Geo g, const float *__restrict__ src, f
 extern "C" int pot3d_gpu_precond_diag(pot3d_gpu_solver *h, float *d, float *dinv) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   Solver &s = h->s;
   if (s.ifprec == 2) return pot3d::dilu_diag(&s, d, dinv);
-  float *tmp = reinterpret_cast<float *>(h->d_io);
+  float *tmp = reinterpret_cast<float *>(s.d_io);
   k_unpack_f<<<pot3d::grid1d(s.g.N), pot3d::NTHR, 0, s.stream>>>(s.g, s.d_ai, tmp);
   CKS(cudaGetLastError());
   if (d) CKS(cudaMemcpyAsync(d, tmp, sizeof(float) * s.g.N, cudaMemcpyDeviceToHost, s.stream));
@@ -261,6 +270,7 @@ extern "C" int pot3d_gpu_precond_diag(pot3d_gpu_solver *h, float *d, float *dinv
 extern "C" int pot3d_gpu_time_kernels(pot3d_gpu_solver *h, int reps, double ms[2], double bytes[2]) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   if (reps <= 0 || h->s.ifprec == 2) {
     pot3d_set_error("time_kernels: reps must be positive and ifprec 0 or 1");
     return POT3D_ERR_ARG;
@@ -271,6 +281,7 @@ extern "C" int pot3d_gpu_time_kernels(pot3d_gpu_solver *h, int reps, double ms[2
 extern "C" int pot3d_gpu_time_sweeps(pot3d_gpu_solver *h, int reps, double ms[2]) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   if (reps <= 0 || h->s.ifprec != 2 || !ms) {
     pot3d_set_error("time_sweeps: reps must be positive and ifprec 2");
     return POT3D_ERR_ARG;
@@ -281,6 +292,7 @@ extern "C" int pot3d_gpu_time_sweeps(pot3d_gpu_solver *h, int reps, double ms[2]
 extern "C" int pot3d_gpu_set_br0(pot3d_gpu_solver *h, const double *br0) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   if (!br0) {
     pot3d_set_error("pot3d_gpu_set_br0: null br0");
     return POT3D_ERR_ARG;
@@ -296,6 +308,7 @@ extern "C" int pot3d_gpu_set_br0(pot3d_gpu_solver *h, const double *br0) {
 extern "C" int pot3d_gpu_set_refine(pot3d_gpu_solver *h, double refine_ratio, double stall_drop, int stall_limit) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   if (!(refine_ratio > 0.0 && refine_ratio < 1.0) || !(stall_drop > 0.0) || stall_limit < 1) {
     pot3d_set_error("pot3d_gpu_set_refine: need 0 < refine_ratio < 1, stall_drop > 0, stall_limit >= 1");
     return POT3D_ERR_ARG;
@@ -316,9 +329,14 @@ extern "C" int pot3d_gpu_refine_info(const pot3d_gpu_solver *h, int *n_refine, i
   return POT3D_OK;
 }
 
+extern "C" int pot3d_gpu_update_group(const pot3d_gpu_solver *h) {
+  return !h ? 0 : h->s.precision == POT3D_FP32_REFINED ? h->s.xg : h->s.xg64;
+}
+
 extern "C" int pot3d_gpu_test_sweep_stall(pot3d_gpu_solver *h, unsigned spin_limit) {
   int st;
   if ((st = check_solver(h))) return st;
+  std::lock_guard<std::mutex> turn(h->turn);
   if (h->s.ifprec != 2 || spin_limit == 0) {
     pot3d_set_error("pot3d_gpu_test_sweep_stall: needs ifprec 2 and a positive spin limit");
     return POT3D_ERR_ARG;

@@ -1388,6 +1388,11 @@ int Solver::setup(const pot3d_mesh_t *mesh, const double *br0, const double *br1
   if ((st = alloc((void **)&d_q, vb))) return st;
   if ((st = alloc((void **)&d_b, vb))) return st;
   if ((st = alloc((void **)&d_tmp, vb))) return st;
+  if (!batched) {  // host vectors' staging
+    const size_t n1 = ((size_t)g.N + 31) / 32 * 32;
+    if ((st = alloc((void **)&d_io, sizeof(double) * (n1 + (size_t)g.N)))) return st;
+    d_io2 = d_io + n1;
+  }
   if ((st = alloc((void **)&d_ai, sizeof(float) * (size_t)g.Np))) return st;
   k_diag_prec<<<grid1d(g.Np), NTHR, 0, stream>>>(g, m, d_ai, ifprec == 0 ? 0 : 1);
   CK(cudaGetLastError());
@@ -1464,60 +1469,44 @@ int Solver::unpack(const double *pad_dev, double *ref_dev) {
 // preconditioner x is updated in groups where the vectors of an iteration
 // outgrow L2 and the update is bound by HBM (121x181x361 FP64: 73 -> 59 us an
 // iteration; 127x181x361 refined: 52 -> 41); below that x stays in L2 and a
-// launch per group costs more than it saves (63x91x181: 11.1 -> 12.9 us).  A
-// rotation that does not fit in memory is left out (groups of two).
+// launch per group costs more than it saves (63x91x181: 11.1 -> 12.9 us).
+// The buffers are vectors that the handle has anyway and that an inner
+// iteration leaves alone, so a rotation takes no memory: d_tmp and the staging
+// of host vectors (FP64), the halves of d_p, d_p2 and d_tmp (refined).  Every
+// valid point of a direction is written before it is read; pad lanes may hold
+// anything, no result depends on them.
 int Solver::x_buffers() {
   if (batched) return POT3D_OK;  // batches update x in pairs from the two buffers
-  int dev = 0, l2 = 0, st;
+  int dev = 0, l2 = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
-  auto more = [&](void **p, size_t bytes) {
-    const int e = alloc(p, bytes);
-    if (e == POT3D_ERR_NOMEM) cudaGetLastError();
-    return e;
-  };
   if (precision == POT3D_FP64) {
-    if (ifprec == 2 || 44LL * g.Np <= l2) return POT3D_OK;  // x, r, p, p', q and a_i
-    m_p64q[0] = d_p;
-    m_p64q[1] = d_p2;
-    xg64 = 2;
-    for (int i = 2; i < X_GROUP64; i++) {
-      if ((st = more((void **)&m_p64q[i], sizeof(double) * (size_t)g.Np)) == POT3D_ERR_NOMEM) return POT3D_OK;
-      if (st) return st;
-    }
+    // x, r, p, p', q and a_i against L2; on grids of fewer than eight radial
+    // points the padded vector can be longer than the staging
+    if (ifprec == 2 || 44LL * g.Np <= l2 || 2 * g.N < g.Np) return POT3D_OK;
+    double *const q[X_GROUP64] = {d_p, d_p2, d_tmp, d_io};
+    std::copy(q, q + X_GROUP64, m_p64q);
     xg64 = X_GROUP64;
     return POT3D_OK;
   }
-  m_p32q[0] = m_p32a;
-  m_p32q[1] = m_p32b;
-  if (ifprec != 2 && 28LL * g.Np <= l2) return POT3D_OK;  // x and FP32 r, p, p', q, a_i
-  xg = 2;
-  for (int i = 2; i < X_GROUP; i++) {
-    if ((st = more((void **)&m_p32q[i], sizeof(float) * (size_t)g.Np)) == POT3D_ERR_NOMEM && ifprec != 2) return POT3D_OK;
-    if (st) return st;
-  }
-  xg = X_GROUP;
+  float *const h[3] = {reinterpret_cast<float *>(d_p), reinterpret_cast<float *>(d_p2), reinterpret_cast<float *>(d_tmp)};
+  float *const q[X_GROUP] = {m_p32a, m_p32b, h[0], h[0] + g.Np, h[1], h[1] + g.Np, h[2], h[2] + g.Np};
+  std::copy(q, q + X_GROUP, m_p32q);
+  if (ifprec == 2 || 28LL * g.Np > l2) xg = X_GROUP;  // x and FP32 r, p, p', q, a_i
   return POT3D_OK;
 }
 
-// x += the n iterations' alpha p, the direction of iteration slot i in buffer
-// (i + 1) % n of the rotation.
-int Solver::launch_x_group(const float *const *dirs32, const double *const *dirs64, int n) {
-  auto go = [&](auto zero, auto gc, const auto *const *dirs) {
-    using T = decltype(zero);
-    constexpr int G = decltype(gc)::value;
-    XDirs<T, G> x;
-    for (int i = 0; i < G; i++) x.p[i] = dirs[(i + 1) % G];
-    if (ifprec != 2) return pot3d_cuda_status(launch_pdl(k_update_x_group<T, G>, dim3(xblocks), dim3(NTHR), 0, stream, g,
-                                                         (const SolveState *)d_state, d_x, x), "k_update_x_group");
-    k_update_x_group<T, G><<<xblocks, NTHR, 0, stream>>>(g, d_state, d_x, x);
-    return pot3d_cuda_status(cudaGetLastError(), "k_update_x_group");
-  };
-  if (dirs32)
-    return n == X_GROUP ? go(0.f, std::integral_constant<int, X_GROUP>{}, dirs32)
-                        : go(0.f, std::integral_constant<int, 2>{}, dirs32);
-  return n == X_GROUP64 ? go(0.0, std::integral_constant<int, X_GROUP64>{}, dirs64)
-                        : go(0.0, std::integral_constant<int, 2>{}, dirs64);
+// x += the group's alpha p, the direction of iteration slot i in buffer i + 1
+// of the rotation (modulo its length).
+template <typename T, int G>
+int Solver::launch_x_group(T *const (&dirs)[G]) {
+  XDirs<T, G> x;
+  for (int i = 0; i < G; i++) x.p[i] = dirs[(i + 1) % G];
+  if (ifprec != 2)
+    return pot3d_cuda_status(launch_pdl(k_update_x_group<T, G>, dim3(xblocks), dim3(NTHR), 0, stream, g,
+                                        (const SolveState *)d_state, d_x, x), "k_update_x_group");
+  k_update_x_group<T, G><<<xblocks, NTHR, 0, stream>>>(g, d_state, d_x, x);
+  return pot3d_cuda_status(cudaGetLastError(), "k_update_x_group");
 }
 
 // One PCG iteration (src/pot3d.F90:4336-4365) at position u of a captured graph.
@@ -1571,7 +1560,7 @@ int Solver::launch_iteration(int u) {
     CK(launch_pdl(k_stencil<MODE_PCG>, grid, dim3(NTHR), StageLayout<MODE_PCG>::smem, stream, mp, g, m, sa));
     CK(launch_pdl(k_update<UPD_ITER, false, false>, gridu, dim3(NTHR), 0, stream, g, m, ua));
     int st;
-    if (xg64 > 1 && u % xg64 == xg64 - 1 && (st = launch_x_group(nullptr, m_p64q, xg64))) return st;
+    if (xg64 > 1 && u % xg64 == xg64 - 1 && (st = launch_x_group(m_p64q))) return st;
   }
   std::swap(p_cur, p_nxt);
   return pot3d_cuda_status(cudaGetLastError(), "launch_iteration");
@@ -1896,7 +1885,7 @@ int Solver::launch_iteration32(int u) {
     // sweeps with r32 -= alpha q, rho, beta and ernorm inside them; the
     // south-ring sums of z
     int st;
-    if (u % xg == xg - 1 && (st = launch_x_group(m_p32q, nullptr, xg))) return st;
+    if (u % xg == xg - 1 && (st = launch_x_group(m_p32q))) return st;
     if ((st = dilu_sweeps_fused(this, m_q32))) return st;
     k_south_ring_z<<<dim3((g.nrm2 + 127) / 128, g.nkc_u), 128, 0, stream>>>(g, m, (const float *)dilu_z32(this), d_s1z);
   } else {
@@ -1905,7 +1894,7 @@ int Solver::launch_iteration32(int u) {
     CK(launch_pdl(k_stencil<MODE_PCG32>, grid, dim3(NTHR), StageLayout<MODE_PCG32>::smem, stream, mp, g, m, sa));
     CK(launch_pdl(k_update<UPD_ITER, false, true>, gridu, dim3(NTHR), 0, stream, g, m, ua));
     int st;
-    if (xg > 1 && u % xg == xg - 1 && (st = launch_x_group(m_p32q, nullptr, xg))) return st;
+    if (xg > 1 && u % xg == xg - 1 && (st = launch_x_group(m_p32q))) return st;
   }
   std::swap(p32_cur, p32_nxt);
   return pot3d_cuda_status(cudaGetLastError(), "launch_iteration32");

@@ -34,8 +34,8 @@ struct Solver {
   int hist_cap = 0;
   // padded FP64 vectors
   double *d_x = nullptr, *d_r = nullptr, *d_p = nullptr, *d_p2 = nullptr, *d_q = nullptr, *d_b = nullptr;
-  double *d_tmp = nullptr;      // scratch (API packing, residual)
-  double *d_ref = nullptr;      // scratch in the reference packed layout (N)
+  double *d_tmp = nullptr;      // scratch (API packing, residual); idle in an iteration
+  double *d_io = nullptr, *d_io2 = nullptr;  // host vectors' staging, reference packed layout (N); idle in a solve
   double *d_phi = nullptr;      // (nr,nt,np) scratch for finalize/energy
   float *d_ai = nullptr;        // diagonal preconditioner (FP32, padded)
   double *p_cur = nullptr, *p_nxt = nullptr;
@@ -43,16 +43,18 @@ struct Solver {
   // FP32-inner / FP64-refined mode (both preconditioners)
   float *m_p32a = nullptr, *m_p32b = nullptr, *m_r32 = nullptr, *m_q32 = nullptr;
   // The search directions of consecutive iterations rotate through xg
-  // buffers, so the solution update is applied once per xg iterations: xg =
-  // X_GROUP (refined) or X_GROUP64 (FP64, diagonal preconditioner), or 2 (the
-  // two buffers every solve has) where the others do not fit in memory; the
-  // FP64 ILU(0) solve updates x every iteration (xg 1).
+  // (refined) or xg64 (FP64) buffers, so the solution update is applied once
+  // per so many iterations: X_GROUP in the refined mode with ILU(0) and, on
+  // grids above L2, with the diagonal preconditioner; X_GROUP64 in FP64 with
+  // the diagonal preconditioner on grids above L2; else 1, the directions
+  // alternate between two buffers and every iteration updates x.
   float *m_p32q[X_GROUP] = {};
   double *m_p64q[X_GROUP64] = {};
   int xg = 1, xg64 = 1;
   bool batched = false;  // a case of a batch (set before setup)
-  int x_buffers();   // allocate the rotation (setup)
-  int launch_x_group(const float *const *dirs32, const double *const *dirs64, int n);
+  int x_buffers();       // choose the rotation (setup)
+  template <typename T, int G>
+  int launch_x_group(T *const (&dirs)[G]);
   float *p32_cur = nullptr, *p32_nxt = nullptr;
   cudaGraphExec_t graph32_exec = nullptr;
   int graph32_U = 0;

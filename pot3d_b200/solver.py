@@ -123,6 +123,10 @@ class Pot3dSolver:
         check(_lib.lib().pot3d_gpu_refine_info(self._h, C.byref(nr), C.byref(fb)))
         return nr.value, fb.value
 
+    def update_group(self) -> int:
+        """Iterations per update of the solution in this handle's solves."""
+        return int(_lib.lib().pot3d_gpu_update_group(self._h))
+
     def test_sweep_stall(self, spin_limit: int = 1 << 12) -> int:
         """Status code of an ILU(0) forward sweep run with one tile left
         undone (POT3D_ERR_TIMEOUT = 6 when its consumers' bounded waits gave
