@@ -515,7 +515,12 @@ __device__ __forceinline__ void stencil_body(const StencilMaps &maps, const Geo 
     // Drain the loads still in flight (bounded), report, and leave.
     if (tid == 0) {
       for (int l = local; l < issued; l++) mbar_wait(&bar[l % S_STAGES], (l / S_STAGES) & 1, WAIT_LIMIT);
-      if (MODE != MODE_AX) atomicExch(&a.st->status, ST_TIMEOUT);
+      if (MODE != MODE_AX) {
+        // no block is the last to arrive now, so nothing else writes the slot,
+        // which still holds an earlier group's alpha
+        if (a.xslot1) a.st->xa[a.xslot1 - 1] = 0.0;
+        atomicExch(&a.st->status, ST_TIMEOUT);
+      }
     }
     return;
   }

@@ -1,6 +1,7 @@
 """Rules of the CUDA source that no run can show to be kept: a kernel launched
 while its predecessor still runs must not read through the read-only path what
-that predecessor writes."""
+that predecessor writes, and an iteration that gives up leaves no step length
+for the grouped solution update."""
 import os
 import re
 
@@ -41,3 +42,11 @@ def test_overlapped_kernels_read_only_setup_data_through_the_read_only_path():
         for par in re.findall(r"const [^,()]*__restrict__[^,()]*", text):
             assert "BatchInst" in par, (k, par)
         assert "ld.global.nc" not in text
+
+
+def test_every_early_exit_of_the_stencil_clears_its_step_length():
+    body = _functions(_source("pcg.cu"))["stencil_body"]
+    exits = [body[:m.start()].rsplit("if (", 2) for m in re.finditer(r"\breturn;", body)]
+    assert len(exits) == 2  # not running any more; a wait that ran out
+    for e in exits:
+        assert re.search(r"if \(a\.xslot1\b[^;]*a\.st->xa\[a\.xslot1 - 1\] = 0\.0;", "if (" + "if (".join(e[1:])), e[1:]
