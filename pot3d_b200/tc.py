@@ -27,13 +27,15 @@ def _fn():
 
 
 def _err_flag(device):
+    """The error flag of a device (a torch.device or its name; without an
+    index, the current one): one int32 that a timed-out wait sets."""
     import torch
-    flag = _err.get(device)
+    i = device.index if isinstance(device, torch.device) else torch.device(device).index
+    if i is None:
+        i = torch.cuda.current_device()
+    flag = _err.get(i)
     if flag is None:
-        key = str(device)
-        if key not in _err:
-            _err[key] = torch.zeros(1, dtype=torch.int32, device=device)
-        flag = _err[device] = _err[key]
+        flag = _err.setdefault(i, torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", i)))
     return flag
 
 

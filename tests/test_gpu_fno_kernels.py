@@ -66,6 +66,21 @@ def test_gemm_split_k_strides_and_act(cuda, b, m, n, k):
     check_errors()
 
 
+def test_a_product_whose_wait_ran_out_is_reported(cuda):
+    import torch
+    from pot3d_b200.tc import _err_flag, check_errors, tc_gemm
+    out = tc_gemm(_t((16, 64), cuda, 17, torch.bfloat16), _t((16, 64), cuda, 18, torch.bfloat16))
+    check_errors()
+    flag = _err_flag(out.device)
+    flag.fill_(1)  # as the kernel does
+    try:
+        with pytest.raises(RuntimeError):
+            check_errors()
+    finally:
+        flag.zero_()
+    check_errors()
+
+
 @pytest.mark.parametrize("b,w,nph,nth", [(1, 32, 3, 33), (2, 17, 5, 31), (1, 64, 2, 96)])
 def test_spec_act(cuda, b, w, nph, nth):
     import torch
