@@ -44,7 +44,8 @@ def raw_stream(device_index):
     some fifty launches, and building torch's stream object for each made the
     host the bound of a guess (1.06 -> 0.91 ms at 255x361x721)."""
     import torch
-    return torch._C._cuda_getCurrentRawStream(device_index)
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # not a public name
+    return raw(device_index) if raw else torch.cuda.current_stream(device_index).cuda_stream
 
 
 def k_splits(batch, M, N, K):

@@ -24,3 +24,9 @@ def test_check_errors_reads_the_flag_that_products_write(one_device, asked):
     with pytest.raises(RuntimeError):
         tc.check_errors()
     tc.check_errors("cuda:0")
+
+
+def test_raw_stream_without_the_private_name(monkeypatch):
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda i: type("Stream", (), {"cuda_stream": 1000 + i})())
+    assert tc.raw_stream(3) == 1003
