@@ -63,6 +63,8 @@ def tc_gemm(A, B, bias=None, out=None, out_dtype=None, ldd=None, accumulate=Fals
     (row stride ldd, e.g. a zero-padded channel buffer).  act "gelu" applies
     the activation to the result."""
     import torch
+    if act not in (None, "gelu"):
+        raise ValueError(f"tc_gemm: unknown activation {act!r}")
     squeeze = A.dim() == 2
     assert A.dtype == torch.bfloat16 and B.dtype == torch.bfloat16 and A.is_cuda and B.is_cuda
     assert A.is_contiguous() and B.is_contiguous()

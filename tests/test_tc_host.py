@@ -30,3 +30,9 @@ def test_raw_stream_without_the_private_name(monkeypatch):
     monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda i: type("Stream", (), {"cuda_stream": 1000 + i})())
     assert tc.raw_stream(3) == 1003
+
+
+def test_unknown_activation_is_refused():
+    a = torch.zeros((16, 64), dtype=torch.bfloat16)
+    with pytest.raises(ValueError):
+        tc.tc_gemm(a, a, act="relu")
