@@ -53,7 +53,7 @@ int pot3d_fno_relmse(const float *pred, int ldp, const void *tgt, int t_dt, int 
                      float scale, float *grad, float *loss, void *stream);
 /* The same with the caller's scratch (device floats, pot3d_fno_relmse_scratch
  * of them) instead of a stream-ordered allocation. */
-int pot3d_fno_relmse_scratch(int nbatch);
+long long pot3d_fno_relmse_scratch(int nbatch);
 int pot3d_fno_relmse_ws(const float *pred, int ldp, const void *tgt, int t_dt, int nbatch, long long npos, int R,
                         float scale, float *grad, float *loss, float *ws, void *stream);
 

@@ -284,19 +284,19 @@ __global__ void k_colsum_final(const float *__restrict__ part, int nb, int C, fl
 
 // Per sample b: loss_b = sum (pred - tgt)^2 / sum tgt^2 over npos x R values;
 // grad = 2 (pred - tgt) / sum tgt^2 * scale.  pred rows have ldp >= R.  Three
-// launches: RM_BLOCKS partial sums a sample, their total in a fixed order, the
-// gradient.  (One block a sample did both passes over a sample's 8 million
+// launches: up to RM_BLOCKS partial sums a sample, their total in a fixed
+// order, the gradient.  The sample is grid.x, which has no limit of 65535.  (One block a sample did both passes over a sample's 8 million
 // values alone: 38 ms for four 127x181x361 samples, against 0.2 ms.)
 constexpr int RM_BLOCKS = 256;
 constexpr int RM_POS = 8;  // positions a block takes at once, one per warp
 __global__ void __launch_bounds__(256) k_relmse_part(const float *__restrict__ pred, int ldp,
                                                      const void *__restrict__ tgt, int t_dt, long long npos, int R,
                                                      float *__restrict__ part) {
-  const int b = blockIdx.y, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int b = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const float *pb = pred + (long long)b * npos * ldp;
   const long long tb = (long long)b * npos * R;
   float se = 0.0f, st2 = 0.0f;
-  for (long long p = (long long)blockIdx.x * RM_POS + w; p < npos; p += (long long)RM_BLOCKS * RM_POS) {
+  for (long long p = (long long)blockIdx.y * RM_POS + w; p < npos; p += (long long)gridDim.y * RM_POS) {
     for (int c = lane; c < R; c += 32) {
       const float tv = ld(tgt, tb + p * R + c, t_dt);
       const float d = pb[p * ldp + c] - tv;
@@ -322,17 +322,20 @@ __global__ void __launch_bounds__(256) k_relmse_part(const float *__restrict__ p
       a += r1[q];
       c += r2[q];
     }
-    part[2 * (b * RM_BLOCKS + blockIdx.x)] = a;
-    part[2 * (b * RM_BLOCKS + blockIdx.x) + 1] = c;
+    const long long q = 2 * ((long long)b * gridDim.y + blockIdx.y);
+    part[q] = a;
+    part[q + 1] = c;
   }
 }
 // den[b] and loss[b] from the sample's partial sums (one warp a sample).
-__global__ void k_relmse_sum(const float *__restrict__ part, float *__restrict__ den, float *__restrict__ loss) {
+__global__ void k_relmse_sum(const float *__restrict__ part, int nblk, float *__restrict__ den,
+                             float *__restrict__ loss) {
   const int b = blockIdx.x, lane = threadIdx.x;
+  const float *pb = part + 2LL * b * nblk;
   float se = 0.0f, st2 = 0.0f;
-  for (int q = lane; q < RM_BLOCKS; q += 32) {
-    se += part[2 * (b * RM_BLOCKS + q)];
-    st2 += part[2 * (b * RM_BLOCKS + q) + 1];
+  for (int q = lane; q < nblk; q += 32) {
+    se += pb[2 * q];
+    st2 += pb[2 * q + 1];
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -349,12 +352,12 @@ __global__ void __launch_bounds__(256) k_relmse_grad(const float *__restrict__ p
                                                      const void *__restrict__ tgt, int t_dt, long long npos, int R,
                                                      float scale, const float *__restrict__ den,
                                                      float *__restrict__ grad) {
-  const int b = blockIdx.y, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int b = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const float *pb = pred + (long long)b * npos * ldp;
   float *gb = grad + (long long)b * npos * ldp;
   const long long tb = (long long)b * npos * R;
   const float f = 2.0f * scale / den[b];
-  for (long long p = (long long)blockIdx.x * RM_POS + w; p < npos; p += (long long)gridDim.x * RM_POS)
+  for (long long p = (long long)blockIdx.y * RM_POS + w; p < npos; p += (long long)gridDim.y * RM_POS)
     for (int c = lane; c < ldp; c += 32)
       gb[p * ldp + c] = c < R ? f * (pb[p * ldp + c] - ld(tgt, tb + p * R + c, t_dt)) : 0.0f;
 }
@@ -505,6 +508,14 @@ extern "C" int pot3d_fno_colsum(const float *in, long long M, int C, int ld, flo
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_colsum");
 }
 
+namespace {
+// Partial sums a sample: a block takes RM_POS positions at least.
+int relmse_blocks(long long npos) {
+  const long long nb = (npos + RM_POS - 1) / RM_POS;
+  return (int)(nb < RM_BLOCKS ? nb : RM_BLOCKS);
+}
+}  // namespace
+
 extern "C" int pot3d_fno_relmse(const float *pred, int ldp, const void *tgt, int t_dt, int nbatch, long long npos,
                                 int R, float scale, float *grad, float *loss, void *stream) {
   if (nbatch < 1 || npos < 1 || R < 1 || ldp < R) {
@@ -513,7 +524,7 @@ extern "C" int pot3d_fno_relmse(const float *pred, int ldp, const void *tgt, int
   }
   float *ws = nullptr;
   cudaStream_t s = (cudaStream_t)stream;
-  const size_t bytes = sizeof(float) * (size_t)pot3d_fno_relmse_scratch(nbatch);
+  const size_t bytes = sizeof(float) * (size_t)nbatch * (2 * relmse_blocks(npos) + 1);
   int st = pot3d_cuda_status(cudaMallocAsync((void **)&ws, bytes, s), "cudaMallocAsync(relmse)");
   if (st) return st;
   st = pot3d_fno_relmse_ws(pred, ldp, tgt, t_dt, nbatch, npos, R, scale, grad, loss, ws, stream);
@@ -521,20 +532,21 @@ extern "C" int pot3d_fno_relmse(const float *pred, int ldp, const void *tgt, int
   return st ? st : fst;
 }
 
-extern "C" int pot3d_fno_relmse_scratch(int nbatch) { return nbatch * (2 * RM_BLOCKS + 1); }
+extern "C" long long pot3d_fno_relmse_scratch(int nbatch) { return (long long)nbatch * (2 * RM_BLOCKS + 1); }
 
 extern "C" int pot3d_fno_relmse_ws(const float *pred, int ldp, const void *tgt, int t_dt, int nbatch, long long npos,
                                    int R, float scale, float *grad, float *loss, float *ws, void *stream) {
-  if (nbatch < 1 || nbatch > 65535 || npos < 1 || R < 1 || ldp < R || !ws) {
+  if (nbatch < 1 || npos < 1 || R < 1 || ldp < R || !ws) {
     pot3d_set_error("pot3d_fno_relmse: bad sizes");
     return POT3D_ERR_ARG;
   }
   cudaStream_t s = (cudaStream_t)stream;
-  float *part = ws, *den = ws + (size_t)nbatch * 2 * RM_BLOCKS;
-  k_relmse_part<<<dim3(RM_BLOCKS, nbatch), 256, 0, s>>>(pred, ldp, tgt, t_dt, npos, R, part);
-  k_relmse_sum<<<nbatch, 32, 0, s>>>(part, den, loss);
+  const int nblk = relmse_blocks(npos);
+  float *den = ws, *part = ws + nbatch;
+  k_relmse_part<<<dim3(nbatch, nblk), 256, 0, s>>>(pred, ldp, tgt, t_dt, npos, R, part);
+  k_relmse_sum<<<nbatch, 32, 0, s>>>(part, nblk, den, loss);
   const long long nb = (npos + RM_POS - 1) / RM_POS;
-  k_relmse_grad<<<dim3((unsigned)(nb < 148 * 16 ? nb : 148 * 16), nbatch), 256, 0, s>>>(pred, ldp, tgt, t_dt, npos, R,
+  k_relmse_grad<<<dim3(nbatch, (unsigned)(nb < 148 * 16 ? nb : 148 * 16)), 256, 0, s>>>(pred, ldp, tgt, t_dt, npos, R,
                                                                                        scale, den, grad);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_relmse");
 }

@@ -53,6 +53,7 @@ def _L():
         L.pot3d_fno_gelu.argtypes = [vp, ll, C.c_int, C.c_int, vp, C.c_int, C.c_int, vp, C.c_int, C.c_int, C.c_int, vp]
         L.pot3d_fno_colsum.argtypes = [vp, ll, C.c_int, C.c_int, vp, C.c_int, vp, C.c_int, vp]
         L.pot3d_fno_relmse_ws.argtypes = [vp, C.c_int, vp, C.c_int, C.c_int, ll, C.c_int, C.c_float, vp, vp, vp, vp]
+        L.pot3d_fno_relmse_scratch.restype = ll
         L.pot3d_fno_spec_act.argtypes = [vp, vp] + [C.c_int] * 7 + [vp, vp]
         L.pot3d_fno_adam.argtypes = [vp, vp, vp, vp, vp, ll, C.c_float, C.c_float, C.c_float, C.c_float, C.c_int, vp]
         L.pot3d_fno_inputs.argtypes = [vp, vp, ll, ll, vp, vp]
