@@ -23,7 +23,7 @@ def _t(shape, cuda, seed=0, dtype=None):
 
 
 @pytest.mark.parametrize("perm", [(0, 1, 3, 2), (0, 3, 1, 2), (0, 2, 3, 1), (2, 3, 0, 1), (0, 1, 2, 3), (3, 0, 1, 2)])
-@pytest.mark.parametrize("dims", [(2, 3, 130, 65), (1, 2, 1, 33), (3, 1, 257, 16)])
+@pytest.mark.parametrize("dims", [(2, 3, 130, 65), (1, 2, 1, 33), (3, 1, 257, 16), (5, 4, 7, 3), (2, 129, 16, 32), (33, 5, 15, 32)])
 def test_permute_pads_crops_and_adds(cuda, perm, dims):
     import torch
     from pot3d_b200.fno import permute
@@ -39,6 +39,25 @@ def test_permute_pads_crops_and_adds(cuda, perm, dims):
         ref = (out.float() + ref if add else ref).to(dt[dst])
         permute(x, dims, out, out_dims, perm, add=add)
         assert torch.equal(out, ref), (src, dst, add)
+
+
+def test_permute_of_short_axes_costs_no_more_than_its_elements(cuda):
+    """The same elements with axes of 1 x 1 and of 64 x 64 to turn; a tile an
+    element took 300 times as long as an element at a time."""
+    import torch
+    from pot3d_b200.fno import permute
+    n, ms = 1 << 23, []
+    x, out = _t((n,), cuda, 19), torch.empty(n, device=cuda)
+    for k in (1, 64):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        for timed in (False, True):
+            e[0].record()
+            permute(x, (1, n // (k * k), k, k), out, (1, n // (k * k), k, k), (0, 1, 3, 2))
+            e[1].record()
+            torch.cuda.synchronize()
+        assert torch.equal(out.view(-1, k, k), x.view(-1, k, k).transpose(1, 2))
+        ms.append(e[0].elapsed_time(e[1]))
+    assert ms[0] < 30 * ms[1], ms
 
 
 @pytest.mark.parametrize("b,m,n,k", [(1, 32, 64, 64 * 67), (1, 128, 128, 64 * 300), (1, 130, 16, 64 * 64),
