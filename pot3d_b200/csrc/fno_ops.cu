@@ -31,6 +31,28 @@ __device__ __forceinline__ void st(void *p, long long i, int dt, float v) {
     reinterpret_cast<__nv_bfloat16 *>(p)[i] = __float2bfloat16_rn(v);
 }
 
+// f(row, column) for every element of rows x cols.  A warp a row spares a
+// division per element, but leaves lanes idle on rows of fewer than 32 columns
+// and the chip on few rows: those go element by element (4.2 million values a
+// GELU: 32 columns 26 us by rows, 1 column 392 by rows and 30 by elements).
+__host__ __device__ inline bool by_elements(long long rows, long long cols) { return cols < 32 || rows < 2048; }
+template <typename F>
+__device__ __forceinline__ void each_element(long long rows, int cols, F f) {
+  const long long n = rows * cols;
+  if (!by_elements(rows, cols)) {
+    for (long long r = blockIdx.x * 8LL + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8LL)
+#pragma unroll 4
+      for (int c = threadIdx.x & 31; c < cols; c += 32) f(r, c);
+  } else if (n < 1LL << 31) {
+    for (unsigned t = blockIdx.x * 256u + threadIdx.x; t < (unsigned)n; t += gridDim.x * 256u) {
+      const unsigned r = t / (unsigned)cols;
+      f((long long)r, (int)(t - r * (unsigned)cols));
+    }
+  } else {
+    for (long long t = blockIdx.x * 256LL + threadIdx.x; t < n; t += gridDim.x * 256LL) f(t / cols, (int)(t % cols));
+  }
+}
+
 struct Dims4 {
   long long d[4];
 };
@@ -83,8 +105,8 @@ __global__ void __launch_bounds__(256) k_permute_rows8(PermArgs a, unsigned n) {
     reinterpret_cast<uint4 *>(a.out)[t] = *reinterpret_cast<const uint4 *>(o);
   }
 }
-// Any permutation, one element at a time: where the axes to be turned are too
-// short for tiles (pot3d_fno_permute).
+// Any permutation, one element at a time: where rows, or the axes to be turned,
+// are too short for the forms around it (pot3d_fno_permute).
 __global__ void __launch_bounds__(256) k_permute_any(PermArgs a, long long n) {
   for (long long t = blockIdx.x * 256LL + threadIdx.x; t < n; t += gridDim.x * 256LL) {
     long long r = t / a.od[3];
@@ -233,16 +255,14 @@ __global__ void __launch_bounds__(256) k_spec_act(float *__restrict__ pre, const
 __global__ void __launch_bounds__(256) k_gelu(const float *__restrict__ pre, long long M, int C, int ldp,
                                               const void *__restrict__ grad, int g_dt, int ldg, void *__restrict__ out,
                                               int out_dt, int ldo, int backward) {
-  const int lane = threadIdx.x & 31;
-  for (long long m = blockIdx.x * 8LL + (threadIdx.x >> 5); m < M; m += gridDim.x * 8LL)
-    for (int c = lane; c < ldo; c += 32) {
-      float v = 0.0f;
-      if (c < C) {
-        const float x = pre[m * ldp + c];
-        v = backward ? ld(grad, m * ldg + c, g_dt) * gelu_d(x) : gelu_f(x);
-      }
-      st(out, m * ldo + c, out_dt, v);
+  each_element(M, ldo, [&](long long m, int c) {
+    float v = 0.0f;
+    if (c < C) {
+      const float x = pre[m * ldp + c];
+      v = backward ? ld(grad, m * ldg + c, g_dt) * gelu_d(x) : gelu_f(x);
     }
+    st(out, m * ldo + c, out_dt, v);
+  });
 }
 
 // out[c] = sum_m in[m][c], c < C: partial sums in a fixed order, 64 blocks of
@@ -422,6 +442,7 @@ int grid_for(long long n) {
   if (b > 148LL * 32) b = 148LL * 32;
   return (int)(b < 1 ? 1 : b);
 }
+int rows_grid(long long rows, long long cols) { return grid_for(rows * (by_elements(rows, cols) ? cols : 32)); }
 
 }  // namespace
 
@@ -457,6 +478,8 @@ extern "C" int pot3d_fno_permute(const void *in, int in_dt, const long long *in_
     if (in_dt == DT_F32 && out_dt == DT_BF16 && !add && a.od[3] % 8 == 0 && a.ie[3] % 4 == 0 && a.is[0] % 4 == 0 &&
         a.is[1] % 4 == 0 && a.is[2] % 4 == 0 && n8 < (1LL << 30) && ((uintptr_t)in | (uintptr_t)out) % 16 == 0)
       k_permute_rows8<<<grid_for(n8), 256, 0, s>>>(a, (unsigned)n8);
+    else if (a.od[3] < 64 || rows < 2048)  // 4.2 million values: 1 column 642 us by rows and 28 by elements, 64 25 and 28
+      k_permute_any<<<grid_for(rows * a.od[3]), 256, 0, s>>>(a, rows * a.od[3]);
     else
       k_permute_rows<<<grid_for(rows * 32), 256, 0, s>>>(a, rows);
   } else {
@@ -508,7 +531,7 @@ extern "C" int pot3d_fno_gelu(const float *pre, long long M, int C, int ldp, con
     pot3d_set_error("pot3d_fno_gelu: bad sizes");
     return POT3D_ERR_ARG;
   }
-  k_gelu<<<grid_for(M * 32), 256, 0, (cudaStream_t)stream>>>(pre, M, C, ldp, grad, g_dt, ldg, out, out_dt, ldo,
+  k_gelu<<<rows_grid(M, ldo), 256, 0, (cudaStream_t)stream>>>(pre, M, C, ldp, grad, g_dt, ldg, out, out_dt, ldo,
                                                                backward);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_gelu");
 }
@@ -598,45 +621,49 @@ namespace {
 // back to the solver's packed FP64 layout (positions (phi, theta), r fastest).
 __global__ void __launch_bounds__(256) k_guess(const float *__restrict__ out, long long B, long long npos, int Rp,
                                                int R, const double *__restrict__ sigma, double *__restrict__ x) {
-  const int lane = threadIdx.x & 31;
-  for (long long bp = blockIdx.x * 8LL + (threadIdx.x >> 5); bp < B * npos; bp += gridDim.x * 8LL) {
-    const double sg = sigma[bp / npos];
-    for (int i = lane; i < R; i += 32) x[bp * R + i] = (double)out[bp * Rp + i] * sg;
-  }
+  each_element(B * npos, R, [&](long long bp, int i) {
+    x[bp * R + i] = (double)out[bp * Rp + i] * sigma[B == 1 ? 0 : bp / npos];
+  });
 }
 // The same with the radial levels resampled: the network's Rs levels (those
 // of the mesh it was trained on) interpolated linearly onto the solver's R
 // levels, level i from source levels idx[i] and idx[i]+1 with weight w[i]
 // (outside [0, 1] at the ends: linear extrapolation).
 // A warp a position: the levels' indices and weights stay in L1.
-// Without the staging, which serves every row length, a row's values are
-// converted to FP64 twice for every output, and conversions issue at a tenth
-// of the FP32 rate; STAGED converts a row once into shared memory, a warp a row
-// (182 -> 150 us for 125 -> 253 levels at 359 x 719 positions; rows of up to 768
-// values, where eight fit 48 KB).
+// Without the staging a row's values are converted to FP64 twice for every
+// output, and conversions issue at a tenth of the FP32 rate; STAGED converts a
+// row once into shared memory, a warp a row (182 -> 150 us for 125 -> 253
+// levels at 359 x 719 positions): where the outputs need at least the row's
+// conversions, for rows of up to 768 values, where eight fit 48 KB.
 template <bool STAGED>
 __global__ void __launch_bounds__(256) k_guess_resampled(const float *__restrict__ out, long long B, long long npos,
                                                          int Rp, int Rs, const int *__restrict__ idx,
                                                          const double *__restrict__ w, int R,
                                                          const double *__restrict__ sigma, double *__restrict__ x) {
+  if (!STAGED) {
+    each_element(B * npos, R, [&](long long bp, int i) {
+      const float *o = out + bp * Rp + idx[i];
+      const double lo = (double)o[0], hi = (double)o[1];
+      x[bp * R + i] = fma(w[i], hi - lo, lo) * sigma[B == 1 ? 0 : bp / npos];
+    });
+    return;
+  }
   extern __shared__ double row_s[];
   const int lane = threadIdx.x & 31;
   double *row = row_s + (threadIdx.x >> 5) * Rs;
   for (long long bp = blockIdx.x * 8LL + (threadIdx.x >> 5); bp < B * npos; bp += gridDim.x * 8LL) {
     const double sg = sigma[bp / npos];
     const float *o = out + bp * Rp;
-    if (STAGED) {
 #pragma unroll 4
-      for (int i = lane; i < Rs; i += 32) row[i] = (double)o[i];
-      __syncwarp();
-    }
+    for (int i = lane; i < Rs; i += 32) row[i] = (double)o[i];
+    __syncwarp();
 #pragma unroll 4
     for (int i = lane; i < R; i += 32) {
       const int q = idx[i];
-      const double lo = STAGED ? row[q] : (double)o[q], hi = STAGED ? row[q + 1] : (double)o[q + 1];
+      const double lo = row[q], hi = row[q + 1];
       x[bp * R + i] = fma(w[i], hi - lo, lo) * sg;
     }
-    if (STAGED) __syncwarp();
+    __syncwarp();
   }
 }
 }  // namespace
@@ -648,12 +675,13 @@ extern "C" int pot3d_fno_guess_resampled(const float *out, long long B, long lon
     pot3d_set_error("pot3d_fno_guess_resampled: bad sizes");
     return POT3D_ERR_ARG;
   }
-  const unsigned blocks = grid_for(B * npos * 32);
   const size_t smem = 8 * sizeof(double) * (size_t)Rs;  // a row for each of the eight warps
-  if (smem <= 48 * 1024)
-    k_guess_resampled<true><<<blocks, 256, smem, (cudaStream_t)stream>>>(out, B, npos, Rp, Rs, idx, w, R, sigma, x);
+  if (smem <= 48 * 1024 && 2LL * R >= Rs && !by_elements(B * npos, R))
+    k_guess_resampled<true><<<grid_for(B * npos * 32), 256, smem, (cudaStream_t)stream>>>(out, B, npos, Rp, Rs, idx, w, R,
+                                                                                          sigma, x);
   else
-    k_guess_resampled<false><<<blocks, 256, 0, (cudaStream_t)stream>>>(out, B, npos, Rp, Rs, idx, w, R, sigma, x);
+    k_guess_resampled<false><<<rows_grid(B * npos, R), 256, 0, (cudaStream_t)stream>>>(out, B, npos, Rp, Rs, idx, w, R,
+                                                                                      sigma, x);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_guess_resampled");
 }
 
@@ -663,6 +691,6 @@ extern "C" int pot3d_fno_guess(const float *out, long long B, long long npos, in
     pot3d_set_error("pot3d_fno_guess: bad sizes");
     return POT3D_ERR_ARG;
   }
-  k_guess<<<grid_for(B * npos * 32), 256, 0, (cudaStream_t)stream>>>(out, B, npos, Rp, R, sigma, x);
+  k_guess<<<rows_grid(B * npos, R), 256, 0, (cudaStream_t)stream>>>(out, B, npos, Rp, R, sigma, x);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_guess");
 }

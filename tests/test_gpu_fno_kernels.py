@@ -186,7 +186,33 @@ def test_permute_rows_eight_columns_a_thread(cuda, rows, cols, out_cols):
     assert torch.equal(permute(x, x.shape, out, out.shape, (1, 0, 2, 3)), ref.transpose(0, 1))
 
 
-@pytest.mark.parametrize("b,npos,rs,r", [(1, 1, 2, 1), (2, 1201, 125, 253), (1, 9, 768, 800), (1, 9, 769, 31)])
+@pytest.mark.parametrize("rows,c,ldo", [(1, 1, 1), (3001, 1, 3), (2047, 40, 64), (2048, 31, 31), (2049, 40, 64), (5, 1000, 1001)])
+def test_gelu_and_guess_of_any_width(cuda, rows, c, ldo):
+    import torch
+    from pot3d_b200 import _lib
+    from pot3d_b200.fno import _L, act
+    pre, grad = _t((rows, c), cuda, 20), _t((rows, c), cuda, 21, torch.bfloat16)
+    x = pre.double().requires_grad_(True)
+    ref = torch.nn.functional.gelu(x, approximate="tanh")
+    (dref,) = torch.autograd.grad(ref, x, grad.double())
+    for mode, want in (("gelu", ref.detach()), ("dgelu", dref)):
+        out = torch.full((rows, ldo), 7.0, device=cuda)
+        act(pre, c, c, out, ldo, mode, grad=grad, ldg=c)
+        # tanh of u to 2 ulp of 1, u's own rounding times u, and a few products
+        assert bool(((out[:, :c].double() - want).abs() <= 32 * EPS32 * (1 + pre.abs().double() ** 3) *
+                     (1 + grad.abs().double())).all()), mode
+        assert not out[:, c:].any()
+    for b in (1, 2):
+        sigma, x0 = _t((b,), cuda, 22, torch.float64), torch.empty((b, rows, c), device=cuda, dtype=torch.float64)
+        y = _t((b, rows, ldo), cuda, 23)
+        _lib.check(_L().pot3d_fno_guess(C.c_void_p(y.data_ptr()), b, rows, ldo, c, C.c_void_p(sigma.data_ptr()),
+                                        C.c_void_p(x0.data_ptr()), None))
+        torch.cuda.synchronize()
+        assert torch.equal(x0, y[..., :c].double() * sigma.view(-1, 1, 1))
+
+
+@pytest.mark.parametrize("b,npos,rs,r", [(1, 1, 2, 1), (2, 1201, 125, 253), (1, 2500, 768, 800), (1, 9, 769, 31),
+                                         (2, 1500, 125, 31), (1, 2100, 125, 62), (3, 800, 70, 33)])
 def test_guess_resampled(cuda, b, npos, rs, r):
     import torch
     from pot3d_b200 import _lib
