@@ -267,40 +267,41 @@ __global__ void __launch_bounds__(256) k_gelu(const float *__restrict__ pre, lon
 
 // out[c] = sum_m in[m][c], c < C: partial sums in a fixed order, 64 blocks of
 // 256 chains of rows (chain t of block b takes rows 256 b + t, then every
-// 256 * 64th) and a binary tree over a block's chains.  A block sums 32
-// columns (a lane a column, so a warp reads a line of a row), a warp eight
-// chains of each; the tree's three widest levels are a thread's own chains.
-constexpr int CS_ROWS = 32;      // chains a block reads at once
-constexpr int CS_CHAINS = 256;   // chains of a block
-__global__ void __launch_bounds__(32 * CS_ROWS) k_colsum(const float *__restrict__ in, long long M, int C, int ld,
-                                                         float *__restrict__ part) {
-  constexpr int NC = CS_CHAINS / CS_ROWS;
-  const int lane = threadIdx.x & 31, y = threadIdx.x >> 5, c = blockIdx.y * 32 + lane;
+// 256 * 64th) and a binary tree over a block's chains.  1024 threads take CB
+// columns (a lane a column, so a warp reads a line of a row, or 32 / CB rows of
+// a few columns) and ROWS chains at once; a thread carries the 256 / ROWS
+// chains that the tree's widest levels join.
+constexpr int CS_CHAINS = 256;
+template <int CB>
+__global__ void __launch_bounds__(1024) k_colsum(const float *__restrict__ in, long long M, int C, int ld,
+                                                 float *__restrict__ part) {
+  constexpr int ROWS = CB >= 4 ? 1024 / CB : CS_CHAINS, NC = CS_CHAINS / ROWS;
+  const int lane = threadIdx.x % CB, y = threadIdx.x / CB, c = blockIdx.y * CB + lane;
   float s[NC] = {};
   if (c < C) {
     const float *p = in + c;
     const long long step = gridDim.x * (long long)CS_CHAINS;
     long long m0 = blockIdx.x * (long long)CS_CHAINS + y;
-#pragma unroll 2
-    for (; m0 + CS_ROWS * (NC - 1) < M; m0 += step) {
+#pragma unroll (16 / NC)
+    for (; m0 + ROWS * (NC - 1) < M; m0 += step) {
       float v[NC];
 #pragma unroll
-      for (int j = 0; j < NC; j++) v[j] = p[(m0 + CS_ROWS * j) * ld];
+      for (int j = 0; j < NC; j++) v[j] = p[(m0 + ROWS * j) * ld];
 #pragma unroll
       for (int j = 0; j < NC; j++) s[j] += v[j];
     }
 #pragma unroll
     for (int j = 0; j < NC; j++)
-      if (m0 + CS_ROWS * j < M) s[j] += p[(m0 + CS_ROWS * j) * ld];
+      if (m0 + ROWS * j < M) s[j] += p[(m0 + ROWS * j) * ld];
   }
 #pragma unroll
   for (int o = NC / 2; o > 0; o >>= 1)
 #pragma unroll
     for (int j = 0; j < o; j++) s[j] += s[j + o];
-  __shared__ float red[CS_ROWS][32];
+  __shared__ float red[ROWS][CB];
   red[y][lane] = s[0];
   __syncthreads();
-  for (int o = CS_ROWS / 2; o > 0; o >>= 1) {
+  for (int o = ROWS / 2; o > 0; o >>= 1) {
     if (y < o) red[y][lane] += red[y + o][lane];
     __syncthreads();
   }
@@ -543,7 +544,13 @@ extern "C" int pot3d_fno_colsum(const float *in, long long M, int C, int ld, flo
     pot3d_set_error("pot3d_fno_colsum: bad sizes or scratch too small");
     return POT3D_ERR_ARG;
   }
-  k_colsum<<<dim3(nb, (C + 31) / 32), 32 * CS_ROWS, 0, (cudaStream_t)stream>>>(in, M, C, ld, scratch);
+  // 4.2 million values in 1, 2, 5 columns: 80, 49, 31 us with 32 lanes for them
+  if (C == 1)
+    k_colsum<1><<<nb, CS_CHAINS, 0, (cudaStream_t)stream>>>(in, M, C, ld, scratch);
+  else if (C <= 8)
+    k_colsum<8><<<nb, 1024, 0, (cudaStream_t)stream>>>(in, M, C, ld, scratch);
+  else
+    k_colsum<32><<<dim3(nb, (C + 31) / 32), 1024, 0, (cudaStream_t)stream>>>(in, M, C, ld, scratch);
   k_colsum_final<<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>(scratch, nb, C, out, add);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_colsum");
 }

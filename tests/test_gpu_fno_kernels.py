@@ -149,7 +149,8 @@ def test_relmse_and_colsum(cuda, b, npos, R, ldp):
     assert bool(((s.double() - ref).abs() <= 4 * EPS32 * np.sqrt(b * npos) * flat[:, :R].double().abs().sum(0) + 1e-30).all())
 
 
-@pytest.mark.parametrize("m,c,ld", [(1, 1, 1), (255, 33, 40), (257, 32, 32), (16384 + 31, 125, 128), (5 * 16384 + 300, 7, 64)])
+@pytest.mark.parametrize("m,c,ld", [(1, 1, 1), (255, 33, 40), (257, 32, 32), (16384 + 31, 125, 128), (5 * 16384 + 300, 7, 64),
+                                    (40 * 16384 + 255, 1, 3), (2 * 16384, 8, 8), (300, 2, 2), (20 * 16384 + 1, 9, 9)])
 def test_colsum_order(cuda, m, c, ld):
     """Bit for bit the stated order: 64 blocks of 256 chains of rows, a binary
     tree over a block's chains, then the blocks one after the other."""
