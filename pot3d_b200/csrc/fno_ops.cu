@@ -316,28 +316,41 @@ __global__ void k_colsum_final(const float *__restrict__ part, int nb, int C, fl
 }
 
 // Per sample b: loss_b = sum (pred - tgt)^2 / sum tgt^2 over npos x R values;
-// grad = 2 (pred - tgt) / sum tgt^2 * scale.  pred rows have ldp >= R.  Three
-// launches: up to RM_BLOCKS partial sums a sample, their total in a fixed
-// order, the gradient.  The sample is grid.x, which has no limit of 65535.  (One block a sample did both passes over a sample's 8 million
-// values alone: 38 ms for four 127x181x361 samples, against 0.2 ms.)
+// grad = 2 (pred - tgt) / sum tgt^2 * scale.  pred rows have ldp >= R.  Large
+// samples in three launches: up to RM_BLOCKS partial sums a sample, their total
+// in a fixed order, the gradient.  (One block a sample did both passes over a
+// sample's 8 million values alone: 38 ms for four 127x181x361 samples, against
+// 0.2 ms.)  Small ones in one, a block a sample (relmse_blocks).  The sample is
+// grid.x, which has no limit of 65535.
 constexpr int RM_BLOCKS = 256;
-constexpr int RM_POS = 8;  // positions a block takes at once, one per warp
-__global__ void __launch_bounds__(256) k_relmse_part(const float *__restrict__ pred, int ldp,
-                                                     const void *__restrict__ tgt, int t_dt, long long npos, int R,
-                                                     float *__restrict__ part) {
-  const int b = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const float *pb = pred + (long long)b * npos * ldp;
-  const long long tb = (long long)b * npos * R;
+constexpr int RM_VALUES = 1024;  // values a block takes at least
+
+// A position's values go to 1 to 32 lanes, as many as they are.
+__host__ __device__ inline int lanes_of(int n) { return n > 16 ? 32 : n > 8 ? 16 : n > 4 ? 8 : n > 2 ? 4 : n > 1 ? 2 : 1; }
+
+// Sums of (pred - tgt)^2 and tgt^2 over a block's positions (a thread's are p0,
+// p0 + step, ...), in every thread of the block.
+template <int NW>
+__device__ __forceinline__ float2 relmse_sums(const float *__restrict__ pb, int ldp, const void *__restrict__ tgt,
+                                              int t_dt, long long tb, long long npos, int R, long long p0,
+                                              long long step) {
+  const int L = lanes_of(R), lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   float se = 0.0f, st2 = 0.0f;
-  for (long long p = (long long)blockIdx.y * RM_POS + w; p < npos; p += (long long)gridDim.y * RM_POS) {
-    for (int c = lane; c < R; c += 32) {
-      const float tv = ld(tgt, tb + p * R + c, t_dt);
-      const float d = pb[p * ldp + c] - tv;
-      se += d * d;
-      st2 += tv * tv;
-    }
+  auto add = [&](long long p, int c) {
+    const float tv = ld(tgt, tb + p * R + c, t_dt);
+    const float d = pb[p * ldp + c] - tv;
+    se += d * d;
+    st2 += tv * tv;
+  };
+  const int c0 = lane & (L - 1);
+  if (R > 32) {
+    for (long long p = p0; p < npos; p += step)
+      for (int c = c0; c < R; c += 32) add(p, c);
+  } else if (c0 < R) {
+#pragma unroll 8
+    for (long long p = p0; p < npos; p += step) add(p, c0);
   }
-  __shared__ float r1[8], r2[8];
+  __shared__ float r1[NW], r2[NW];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     se += __shfl_xor_sync(0xffffffffu, se, o);
@@ -348,17 +361,43 @@ __global__ void __launch_bounds__(256) k_relmse_part(const float *__restrict__ p
     r2[w] = st2;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float a = 0.0f, c = 0.0f;
+  float a = 0.0f, c = 0.0f;
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-      a += r1[q];
-      c += r2[q];
-    }
-    const long long q = 2 * ((long long)b * gridDim.y + blockIdx.y);
-    part[q] = a;
-    part[q + 1] = c;
+  for (int q = 0; q < NW; q++) {
+    a += r1[q];
+    c += r2[q];
   }
+  return make_float2(a, c);
+}
+__device__ __forceinline__ void relmse_grad(const float *__restrict__ pb, int ldp, const void *__restrict__ tgt,
+                                            int t_dt, long long tb, long long npos, int R, float f,
+                                            float *__restrict__ gb, long long p0, long long step) {
+  const int c0 = threadIdx.x & (lanes_of(ldp) - 1);
+  auto put = [&](long long p, int c) {
+    gb[p * ldp + c] = c < R ? f * (pb[p * ldp + c] - ld(tgt, tb + p * R + c, t_dt)) : 0.0f;
+  };
+  if (ldp > 32) {
+    for (long long p = p0; p < npos; p += step)
+      for (int c = c0; c < ldp; c += 32) put(p, c);
+  } else if (c0 < ldp) {
+#pragma unroll 4
+    for (long long p = p0; p < npos; p += step) put(p, c0);
+  }
+}
+// The position that a thread of block `blk` of NW warps starts from.
+template <int NW>
+__device__ __forceinline__ long long first_position(int n, unsigned blk) {
+  const int L = lanes_of(n);
+  return (long long)blk * (NW * (32 / L)) + threadIdx.x / L;
+}
+
+__global__ void __launch_bounds__(256) k_relmse_part(const float *__restrict__ pred, int ldp,
+                                                     const void *__restrict__ tgt, int t_dt, long long npos, int R,
+                                                     float *__restrict__ part) {
+  const int b = blockIdx.x;
+  const float2 s = relmse_sums<8>(pred + (long long)b * npos * ldp, ldp, tgt, t_dt, (long long)b * npos * R, npos, R,
+                                  first_position<8>(R, blockIdx.y), (long long)gridDim.y * 8 * (32 / lanes_of(R)));
+  if (threadIdx.x == 0) *reinterpret_cast<float2 *>(part + 2 * ((long long)b * gridDim.y + blockIdx.y)) = s;
 }
 // den[b] and loss[b] from the sample's partial sums (one warp a sample).
 __global__ void k_relmse_sum(const float *__restrict__ part, int nblk, float *__restrict__ den,
@@ -385,14 +424,25 @@ __global__ void __launch_bounds__(256) k_relmse_grad(const float *__restrict__ p
                                                      const void *__restrict__ tgt, int t_dt, long long npos, int R,
                                                      float scale, const float *__restrict__ den,
                                                      float *__restrict__ grad) {
-  const int b = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int b = blockIdx.x;
+  relmse_grad(pred + (long long)b * npos * ldp, ldp, tgt, t_dt, (long long)b * npos * R, npos, R, 2.0f * scale / den[b],
+              grad + (long long)b * npos * ldp, first_position<8>(ldp, blockIdx.y),
+              (long long)gridDim.y * 8 * (32 / lanes_of(ldp)));
+}
+// A whole sample: both sums, the loss and the gradient.
+template <int NW>
+__global__ void __launch_bounds__(32 * NW) k_relmse_one(const float *__restrict__ pred, int ldp,
+                                                        const void *__restrict__ tgt, int t_dt, long long npos, int R,
+                                                        float scale, float *__restrict__ grad,
+                                                        float *__restrict__ loss) {
+  const int b = blockIdx.x;
   const float *pb = pred + (long long)b * npos * ldp;
-  float *gb = grad + (long long)b * npos * ldp;
   const long long tb = (long long)b * npos * R;
-  const float f = 2.0f * scale / den[b];
-  for (long long p = (long long)blockIdx.y * RM_POS + w; p < npos; p += (long long)gridDim.y * RM_POS)
-    for (int c = lane; c < ldp; c += 32)
-      gb[p * ldp + c] = c < R ? f * (pb[p * ldp + c] - ld(tgt, tb + p * R + c, t_dt)) : 0.0f;
+  const float2 s = relmse_sums<NW>(pb, ldp, tgt, t_dt, tb, npos, R, first_position<NW>(R, 0), NW * (32 / lanes_of(R)));
+  const float d = fmaxf(s.y, 1e-30f);
+  if (threadIdx.x == 0) loss[b] = s.x / d;
+  relmse_grad(pb, ldp, tgt, t_dt, tb, npos, R, 2.0f * scale / d, grad + (long long)b * npos * ldp,
+              first_position<NW>(ldp, 0), NW * (32 / lanes_of(ldp)));
 }
 
 __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m1, float *__restrict__ m2,
@@ -556,10 +606,23 @@ extern "C" int pot3d_fno_colsum(const float *in, long long M, int C, int ld, flo
 }
 
 namespace {
-// Partial sums a sample: a block takes RM_POS positions at least.
-int relmse_blocks(long long npos) {
-  const long long nb = (npos + RM_POS - 1) / RM_POS;
+// Partial sums a sample: a block takes RM_VALUES values at least.
+int relmse_blocks(long long npos, int R) {
+  const long long nb = (npos * R + RM_VALUES - 1) / RM_VALUES;
   return (int)(nb < RM_BLOCKS ? nb : RM_BLOCKS);
+}
+// More samples than two blocks of 1024 threads an SM: a block of 256 each, all
+// of them in flight (512 samples of 8192 values: 41 us with 1024).
+constexpr int RM_MANY = 296;
+// Without a workspace, samples of up to this many values take a block each: an
+// allocation costs as much as a block takes for so many (see pot3d_fno_relmse).
+constexpr long long RM_ONE = 1 << 17;
+void relmse_one(const float *pred, int ldp, const void *tgt, int t_dt, int nbatch, long long npos, int R, float scale,
+                float *grad, float *loss, cudaStream_t s) {
+  if (npos * ldp <= 4 * RM_VALUES || nbatch > RM_MANY)
+    k_relmse_one<8><<<nbatch, 256, 0, s>>>(pred, ldp, tgt, t_dt, npos, R, scale, grad, loss);
+  else
+    k_relmse_one<32><<<nbatch, 1024, 0, s>>>(pred, ldp, tgt, t_dt, npos, R, scale, grad, loss);
 }
 }  // namespace
 
@@ -569,9 +632,13 @@ extern "C" int pot3d_fno_relmse(const float *pred, int ldp, const void *tgt, int
     pot3d_set_error("pot3d_fno_relmse: bad sizes");
     return POT3D_ERR_ARG;
   }
-  float *ws = nullptr;
   cudaStream_t s = (cudaStream_t)stream;
-  const size_t bytes = sizeof(float) * (size_t)nbatch * (2 * relmse_blocks(npos) + 1);
+  if (npos * R <= RM_ONE || nbatch > RM_MANY) {
+    relmse_one(pred, ldp, tgt, t_dt, nbatch, npos, R, scale, grad, loss, s);
+    return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_relmse");
+  }
+  float *ws = nullptr;
+  const size_t bytes = sizeof(float) * (size_t)nbatch * (2 * relmse_blocks(npos, R) + 1);
   int st = pot3d_cuda_status(cudaMallocAsync((void **)&ws, bytes, s), "cudaMallocAsync(relmse)");
   if (st) return st;
   st = pot3d_fno_relmse_ws(pred, ldp, tgt, t_dt, nbatch, npos, R, scale, grad, loss, ws, stream);
@@ -588,11 +655,15 @@ extern "C" int pot3d_fno_relmse_ws(const float *pred, int ldp, const void *tgt, 
     return POT3D_ERR_ARG;
   }
   cudaStream_t s = (cudaStream_t)stream;
-  const int nblk = relmse_blocks(npos);
-  float *den = ws, *part = ws + nbatch;
+  const int nblk = relmse_blocks(npos, R);
+  if (nblk < 8 || nbatch > RM_MANY) {
+    relmse_one(pred, ldp, tgt, t_dt, nbatch, npos, R, scale, grad, loss, s);
+    return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_relmse");
+  }
+  float *part = ws, *den = ws + (size_t)nbatch * 2 * nblk;
   k_relmse_part<<<dim3(nbatch, nblk), 256, 0, s>>>(pred, ldp, tgt, t_dt, npos, R, part);
   k_relmse_sum<<<nbatch, 32, 0, s>>>(part, nblk, den, loss);
-  const long long nb = (npos + RM_POS - 1) / RM_POS;
+  const long long nb = (npos * ldp + RM_VALUES - 1) / RM_VALUES;
   k_relmse_grad<<<dim3(nbatch, (unsigned)(nb < 148 * 16 ? nb : 148 * 16)), 256, 0, s>>>(pred, ldp, tgt, t_dt, npos, R,
                                                                                        scale, den, grad);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_relmse");

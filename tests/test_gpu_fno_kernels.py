@@ -118,7 +118,8 @@ def test_spec_act(cuda, b, w, nph, nth):
 
 
 @pytest.mark.parametrize("b,npos,R,ldp", [(1, 1, 1, 64), (3, 2049, 125, 128), (2, 70000, 61, 64),
-                                           (70000, 1, 3, 4), (65537, 9, 1, 1)])
+                                           (70000, 1, 3, 4), (65537, 9, 1, 1), (3, 4096, 1, 1),
+                                           (2, 2000, 5, 9), (64, 1030, 17, 20), (1, 1 << 17, 1, 2)])
 def test_relmse_and_colsum(cuda, b, npos, R, ldp):
     import torch
     from pot3d_b200 import _lib
