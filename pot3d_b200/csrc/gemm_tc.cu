@@ -333,32 +333,48 @@ extern "C" int pot3d_tc_gemm(const void *A, const void *B, void *D, const float 
 }
 
 namespace {
-// D (+)= the splits' partial products (+ bias), summed in a fixed order: a
-// block takes 32 outputs, 32 threads an output.
-__global__ void __launch_bounds__(1024) k_splitk_sum(const float *__restrict__ ws, int splits, long long mn, int M, int N,
-                                                     int batch, const float *__restrict__ bias, float *__restrict__ D,
-                                                     long long ldd, long long bstride_d, int accumulate, int act) {
-  const long long n = mn * batch, t = blockIdx.x * 32LL + (threadIdx.x & 31);
+// D (+)= the splits' partial products (+ bias), summed in a fixed order.
+struct SplitSum {
+  const float *ws, *bias;
+  float *D;
+  long long mn, n, ldd, bstride_d;  // n: outputs of all batches
+  int splits, M, N, accumulate, act;
+};
+__device__ __forceinline__ void split_out(const SplitSum &a, long long t, float s) {
+  const int col = (int)(t % a.N);
+  const long long row = t / a.N % a.M, b = t / a.mn;
+  if (a.bias) s += a.bias[col];
+  if (a.act) s = gelu_f(s);
+  float *d = a.D + b * a.bstride_d + row * a.ldd + col;
+  *d = a.accumulate ? *d + s : s;
+}
+// Many splits of few outputs: a block takes 32 outputs, 32 threads an output.
+__global__ void __launch_bounds__(1024) k_splitk_sum(const __grid_constant__ SplitSum a) {
+  const long long t = blockIdx.x * 32LL + (threadIdx.x & 31);
   const int y = threadIdx.x >> 5;
   float s = 0.0f;
-  if (t < n) {
+  if (t < a.n) {
 #pragma unroll 4
-    for (int q = y; q < splits; q += 32) s += ws[q * n + t];
+    for (int q = y; q < a.splits; q += 32) s += a.ws[q * a.n + t];
   }
   __shared__ float red[32][32];
   red[y][threadIdx.x & 31] = s;
   __syncthreads();
-  if (y == 0 && t < n) {
+  if (y == 0 && t < a.n) {
     s = 0.0f;
 #pragma unroll
     for (int q = 0; q < 32; q++) s += red[q][threadIdx.x];
-    const int col = (int)(t % N);
-    const long long row = t / N % M, b = t / mn;
-    if (bias) s += bias[col];
-    if (act) s = gelu_f(s);
-    float *d = D + b * bstride_d + row * ldd + col;
-    *d = accumulate ? *d + s : s;
+    split_out(a, t, s);
   }
+}
+// Up to 32 splits: a thread an output, the same order.
+__global__ void __launch_bounds__(256) k_splitk_sum_few(const __grid_constant__ SplitSum a) {
+  const long long t = blockIdx.x * 256LL + threadIdx.x;
+  if (t >= a.n) return;
+  float s = 0.0f;
+#pragma unroll 8
+  for (int q = 0; q < a.splits; q++) s += a.ws[q * a.n + t];
+  split_out(a, t, s);
 }
 }  // namespace
 
@@ -403,8 +419,10 @@ extern "C" int pot3d_tc_gemm_ex(const void *A, const void *B, void *D, const flo
   POT3D_GEMM_CASE(128)
 #undef POT3D_GEMM_CASE
   if (st || !split) return st;
-  const long long n = mn * batch;
-  k_splitk_sum<<<(unsigned)((n + 31) / 32), 1024, 0, s>>>(ws, splits, mn, M, N, batch, bias,
-                                                          reinterpret_cast<float *>(D), ldd, bstride_d, accumulate, act);
+  const SplitSum a{ws, bias, reinterpret_cast<float *>(D), mn, mn * batch, ldd, bstride_d, splits, M, N, accumulate, act};
+  if (splits <= 32)  // 74 products of 128 x 128 in 4 parts: 72 us, 240 by k_splitk_sum
+    k_splitk_sum_few<<<(unsigned)((a.n + 255) / 256), 256, 0, s>>>(a);
+  else
+    k_splitk_sum<<<(unsigned)((a.n + 31) / 32), 1024, 0, s>>>(a);
   return pot3d_cuda_status(cudaGetLastError(), "k_splitk_sum");
 }

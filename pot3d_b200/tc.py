@@ -50,12 +50,14 @@ def raw_stream(device_index):
 
 def k_splits(batch, M, N, K):
     """Blocks that share the K of one output tile: a product with fewer tiles
-    than half the SMs and a K of 64 or more steps is split so that about two
+    than half the SMs and a K of 64 or more steps, and of two or more a tile
+    (the partial sums cost a pass over all tiles: 74 tiles of 64 steps 72 us
+    split and 62 whole, of 256 steps 143 and 160), is split so that about two
     blocks an SM have work, each with at least 8 steps."""
     tile_n = 32 if N <= 32 else 64 if N <= 64 else 128
     tiles = batch * -(-M // 128) * -(-N // tile_n)
     steps = K // 64
-    return max(1, min(steps // 8, -(-296 // tiles))) if tiles <= 74 and steps >= 64 else 1
+    return max(1, min(steps // 8, -(-296 // tiles))) if tiles <= 74 and steps >= max(64, 2 * tiles) else 1
 
 
 def tc_gemm(A, B, bias=None, out=None, out_dtype=None, ldd=None, accumulate=False, n=None, act=None):

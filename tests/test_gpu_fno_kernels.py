@@ -61,7 +61,7 @@ def test_permute_of_short_axes_costs_no_more_than_its_elements(cuda):
 
 
 @pytest.mark.parametrize("b,m,n,k", [(1, 32, 64, 64 * 67), (1, 128, 128, 64 * 300), (1, 130, 16, 64 * 64),
-                                     (2, 32, 32, 64 * 65), (1, 1000, 48, 64)])
+                                     (2, 32, 32, 64 * 65), (1, 1000, 48, 64), (33, 16, 16, 64 * 67), (30, 100, 16, 64 * 80)])
 def test_gemm_split_k_strides_and_act(cuda, b, m, n, k):
     import torch
     from pot3d_b200.tc import check_errors, k_splits, tc_gemm
@@ -70,7 +70,7 @@ def test_gemm_split_k_strides_and_act(cuda, b, m, n, k):
     mag = A.double().abs() @ B.double().abs().transpose(1, 2) + bias.double().abs()
     tol = 4 * EPS32 * np.sqrt(k) * mag
     splits = k_splits(b, m, n, k)
-    assert (splits > 1) == (k >= 64 * 64)
+    assert (splits > 1) == (k >= 64 * 64 and b * -(-m // 128) * 2 <= k // 64)
     assert bool(((tc_gemm(A, B, bias=bias).double() - ref).abs() <= tol).all())
     acc = _t((b, m, n), cuda, 6)
     got = tc_gemm(A, B, bias=bias, out=acc.clone(), accumulate=True)
