@@ -51,8 +51,8 @@ int pot3d_fno_colsum(const float *in, long long M, int C, int ld, float *out, in
  * gradient scaled by `scale`. */
 int pot3d_fno_relmse(const float *pred, int ldp, const void *tgt, int t_dt, int nbatch, long long npos, int R,
                      float scale, float *grad, float *loss, void *stream);
-/* The same with the caller's scratch (device floats, pot3d_fno_relmse_scratch
- * of them) instead of a stream-ordered allocation. */
+/* The same, faster for few large samples, with the caller's scratch (device
+ * floats, pot3d_fno_relmse_scratch of them). */
 long long pot3d_fno_relmse_scratch(int nbatch);
 int pot3d_fno_relmse_ws(const float *pred, int ldp, const void *tgt, int t_dt, int nbatch, long long npos, int R,
                         float scale, float *grad, float *loss, float *ws, void *stream);

@@ -8,6 +8,7 @@
 //   pot3d_fno_colsum   deterministic column sums (bias gradients)
 //   pot3d_fno_relmse   per-sample relative squared error and its gradient
 //   pot3d_fno_adam     Adam step on FP32 master weights with a BF16 copy
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -320,8 +321,9 @@ __global__ void k_colsum_final(const float *__restrict__ part, int nb, int C, fl
 // samples in three launches: up to RM_BLOCKS partial sums a sample, their total
 // in a fixed order, the gradient.  (One block a sample did both passes over a
 // sample's 8 million values alone: 38 ms for four 127x181x361 samples, against
-// 0.2 ms.)  Small ones in one, a block a sample (relmse_blocks).  The sample is
-// grid.x, which has no limit of 65535.
+// 0.2 ms.)  Small ones, and all of them without a workspace, in one: a block or
+// a cluster of eight a sample (relmse_one).  The sample is grid.x, which has no
+// limit of 65535.
 constexpr int RM_BLOCKS = 256;
 constexpr int RM_VALUES = 1024;  // values a block takes at least
 
@@ -429,20 +431,36 @@ __global__ void __launch_bounds__(256) k_relmse_grad(const float *__restrict__ p
               grad + (long long)b * npos * ldp, first_position<8>(ldp, blockIdx.y),
               (long long)gridDim.y * 8 * (32 / lanes_of(ldp)));
 }
-// A whole sample: both sums, the loss and the gradient.
+// A whole sample, by a block or a cluster: both sums (over the cluster's blocks
+// in order, read from their shared memory), the loss and the gradient.
 template <int NW>
 __global__ void __launch_bounds__(32 * NW) k_relmse_one(const float *__restrict__ pred, int ldp,
                                                         const void *__restrict__ tgt, int t_dt, long long npos, int R,
                                                         float scale, float *__restrict__ grad,
                                                         float *__restrict__ loss) {
-  const int b = blockIdx.x;
-  const float *pb = pred + (long long)b * npos * ldp;
-  const long long tb = (long long)b * npos * R;
-  const float2 s = relmse_sums<NW>(pb, ldp, tgt, t_dt, tb, npos, R, first_position<NW>(R, 0), NW * (32 / lanes_of(R)));
+  const auto cluster = cooperative_groups::this_cluster();
+  const unsigned nc = cluster.num_blocks(), rank = cluster.block_rank();
+  const long long b = blockIdx.x / nc;
+  const float *pb = pred + b * npos * ldp;
+  const long long tb = b * npos * R;
+  __shared__ float2 mine;
+  float2 s = relmse_sums<NW>(pb, ldp, tgt, t_dt, tb, npos, R, first_position<NW>(R, rank),
+                             (long long)nc * NW * (32 / lanes_of(R)));
+  if (nc > 1) {
+    if (threadIdx.x == 0) mine = s;
+    cluster.sync();
+    s = make_float2(0.0f, 0.0f);
+    for (unsigned q = 0; q < nc; q++) {
+      const float2 o = *cluster.map_shared_rank(&mine, q);
+      s.x += o.x;
+      s.y += o.y;
+    }
+    cluster.sync();
+  }
   const float d = fmaxf(s.y, 1e-30f);
-  if (threadIdx.x == 0) loss[b] = s.x / d;
-  relmse_grad(pb, ldp, tgt, t_dt, tb, npos, R, 2.0f * scale / d, grad + (long long)b * npos * ldp,
-              first_position<NW>(ldp, 0), NW * (32 / lanes_of(ldp)));
+  if (rank == 0 && threadIdx.x == 0) loss[b] = s.x / d;
+  relmse_grad(pb, ldp, tgt, t_dt, tb, npos, R, 2.0f * scale / d, grad + b * npos * ldp, first_position<NW>(ldp, rank),
+              (long long)nc * NW * (32 / lanes_of(ldp)));
 }
 
 __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m1, float *__restrict__ m2,
@@ -612,17 +630,27 @@ int relmse_blocks(long long npos, int R) {
   return (int)(nb < RM_BLOCKS ? nb : RM_BLOCKS);
 }
 // More samples than two blocks of 1024 threads an SM: a block of 256 each, all
-// of them in flight (512 samples of 8192 values: 41 us with 1024).
+// of them in flight (512 samples of 8192 values: 41 us with 1024, 24 with 256).
 constexpr int RM_MANY = 296;
-// Without a workspace, samples of up to this many values take a block each: an
-// allocation costs as much as a block takes for so many (see pot3d_fno_relmse).
-constexpr long long RM_ONE = 1 << 17;
-void relmse_one(const float *pred, int ldp, const void *tgt, int t_dt, int nbatch, long long npos, int R, float scale,
-                float *grad, float *loss, cudaStream_t s) {
-  if (npos * ldp <= 4 * RM_VALUES || nbatch > RM_MANY)
+int relmse_one(const float *pred, int ldp, const void *tgt, int t_dt, int nbatch, long long npos, int R, float scale,
+               float *grad, float *loss, cudaStream_t s) {
+  if (npos * ldp <= 4 * RM_VALUES || nbatch > RM_MANY) {
     k_relmse_one<8><<<nbatch, 256, 0, s>>>(pred, ldp, tgt, t_dt, npos, R, scale, grad, loss);
-  else
-    k_relmse_one<32><<<nbatch, 1024, 0, s>>>(pred, ldp, tgt, t_dt, npos, R, scale, grad, loss);
+    return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_relmse");
+  }
+  const unsigned nc = npos * ldp <= 32 * RM_VALUES ? 1 : 8;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(nbatch * nc);
+  cfg.blockDim = dim3(1024);
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = nc;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return pot3d_cuda_status(cudaLaunchKernelEx(&cfg, k_relmse_one<32>, pred, ldp, tgt, t_dt, npos, R, scale, grad, loss),
+                           "pot3d_fno_relmse");
 }
 }  // namespace
 
@@ -632,18 +660,7 @@ extern "C" int pot3d_fno_relmse(const float *pred, int ldp, const void *tgt, int
     pot3d_set_error("pot3d_fno_relmse: bad sizes");
     return POT3D_ERR_ARG;
   }
-  cudaStream_t s = (cudaStream_t)stream;
-  if (npos * R <= RM_ONE || nbatch > RM_MANY) {
-    relmse_one(pred, ldp, tgt, t_dt, nbatch, npos, R, scale, grad, loss, s);
-    return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_relmse");
-  }
-  float *ws = nullptr;
-  const size_t bytes = sizeof(float) * (size_t)nbatch * (2 * relmse_blocks(npos, R) + 1);
-  int st = pot3d_cuda_status(cudaMallocAsync((void **)&ws, bytes, s), "cudaMallocAsync(relmse)");
-  if (st) return st;
-  st = pot3d_fno_relmse_ws(pred, ldp, tgt, t_dt, nbatch, npos, R, scale, grad, loss, ws, stream);
-  const int fst = pot3d_cuda_status(cudaFreeAsync(ws, s), "cudaFreeAsync(relmse)");
-  return st ? st : fst;
+  return relmse_one(pred, ldp, tgt, t_dt, nbatch, npos, R, scale, grad, loss, (cudaStream_t)stream);
 }
 
 extern "C" long long pot3d_fno_relmse_scratch(int nbatch) { return (long long)nbatch * (2 * RM_BLOCKS + 1); }
@@ -656,10 +673,7 @@ extern "C" int pot3d_fno_relmse_ws(const float *pred, int ldp, const void *tgt, 
   }
   cudaStream_t s = (cudaStream_t)stream;
   const int nblk = relmse_blocks(npos, R);
-  if (nblk < 8 || nbatch > RM_MANY) {
-    relmse_one(pred, ldp, tgt, t_dt, nbatch, npos, R, scale, grad, loss, s);
-    return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_relmse");
-  }
+  if (nblk < 8 || nbatch > RM_MANY) return relmse_one(pred, ldp, tgt, t_dt, nbatch, npos, R, scale, grad, loss, s);
   float *part = ws, *den = ws + (size_t)nbatch * 2 * nblk;
   k_relmse_part<<<dim3(nbatch, nblk), 256, 0, s>>>(pred, ldp, tgt, t_dt, npos, R, part);
   k_relmse_sum<<<nbatch, 32, 0, s>>>(part, nblk, den, loss);
