@@ -54,16 +54,23 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "solve s to 1e-9 resid: learned+FP32-refined vs plain FP64 PCG on 1 B200; HBM GB/s"
-# Algorithmic DRAM bytes per unknown (matrix-free coefficients, each vector
-# touched once per fused pass): FP64 PCG iteration 80 (ifprec=1) / 104
-# (ifprec=2); FP32-inner iteration 40 / 64; each FP64 reliable update 24.
-# The ILU(0) application moves 12 B forward (r32, d, y) and 12 B backward
-# (y, d, z32).  In the refined mode's inner iteration the forward sweep also
-# applies the residual half of the update (q32 read, r32 written: +8 B; its
-# r32 read is the sweep's own) and the backward sweep forms rho = r.z (r32
-# read: +4 B; z is its own output).
-BYTES_PER_UNKNOWN_ITER = {("fp64", 1): 80.0, ("fp64", 2): 104.0, ("fp32_refined", 1): 40.0,
-                          ("fp32_refined", 2): 64.0}
+# Algorithmic DRAM bytes per unknown and iteration (matrix-free coefficients and
+# a_i not counted, each vector touched once per fused pass) without x, which is
+# read and written once per group of iterations (16 B, Pot3dSolver.update_group):
+# FP64 64 (ifprec=1) / 88 (ifprec=2); FP32-inner 32 / 56.  Each FP64 reliable
+# update moves 24 more.  The ILU(0) application moves 12 B forward (r32, d, y)
+# and 12 B backward (y, d, z32).  In the refined mode's inner iteration the
+# forward sweep also applies the residual half of the update (q32 read, r32
+# written: +8 B; its r32 read is the sweep's own) and the backward sweep forms
+# rho = r.z (r32 read: +4 B; z is its own output).
+BYTES_PER_UNKNOWN_ITER = {("fp64", 1): 64.0, ("fp64", 2): 88.0, ("fp32_refined", 1): 32.0,
+                          ("fp32_refined", 2): 56.0}
+
+
+def bytes_per_iteration(precision, ifprec, update_group):
+    return BYTES_PER_UNKNOWN_ITER[(precision, 2 if ifprec == 2 else 1)] + 16.0 / update_group
+
+
 BYTES_PER_REFINE = 24.0
 SWEEP_BYTES_PER_UNKNOWN = {"k_dilu_wave<fwd>": 12.0, "k_dilu_wave<bwd>": 12.0,
                            "k_dilu_wave<fwd,fused>": 20.0, "k_dilu_wave<bwd,fused>": 16.0}
@@ -601,13 +608,14 @@ def main():
     if not args.no_plain:
         sp = Pot3dSolver(mesh, br0, option=opt, ifprec=1, precision="fp64", device=local)
         pt = [solve_resident(sp, learned=False) for _ in range(2 if args.warmup > 0 else 1)]
+        plain_bytes = bytes_per_iteration("fp64", 1, sp.update_group())
         sp.close()
         if any(q["ierr"] for q in pt):
             raise SystemExit("the plain FP64 solve did not converge")
         t_plain = reduce_max(pt[-1]["seconds"], ws)
         plain = {"seconds": t_plain, "iterations": pt[-1]["ncg"], "ifprec": 1, "precision": "fp64",
                  "initial_guess": "zero", "speedup": t_plain / t_dev,
-                 "achieved_gbs": 80.0 * N * pt[-1]["ncg"] / t_plain / 1e9}
+                 "achieved_gbs": plain_bytes * N * pt[-1]["ncg"] / t_plain / 1e9}
 
     if rank != 0:
         s.close()
@@ -615,7 +623,7 @@ def main():
     peak, psrc = peak_hbm()
     ncg = int(np.median([q["ncg"] for q in steps]))
     nref = int(np.median([q["n_refine"] for q in steps]))
-    algo_bytes = BYTES_PER_UNKNOWN_ITER[(args.precision, 2 if args.ifprec == 2 else 1)] * N * ncg + \
+    algo_bytes = bytes_per_iteration(args.precision, args.ifprec, s.update_group()) * N * ncg + \
         BYTES_PER_REFINE * N * nref
     overall_gbs = algo_bytes / t_dev / 1e9
     roofline = None

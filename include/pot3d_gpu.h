@@ -205,10 +205,13 @@ int pot3d_gpu_precond_diag(pot3d_gpu_solver *s, float *d, float *dinv);
 
 /* Times the two kernels of one FP64 PCG iteration with CUDA events on the
  * solver's stream: reps iterations from a fresh start (r = b, p = 0), the
- * stencil+dot kernel and the update+dot kernel timed separately.
- * ms[0], ms[1] = average milliseconds per launch; bytes[0], bytes[1] = the
- * algorithmic DRAM bytes per launch (stencil: r, p read, p, Ap written;
- * update: x, p, r, Ap read, x, r written; 8 B each per unknown). */
+ * stencil+dot kernel and the update+dot kernel timed separately, the latter
+ * with its share of the grouped update of x where there is one
+ * (pot3d_gpu_update_group; reps is rounded up to whole groups).
+ * ms[0], ms[1] = average milliseconds per iteration; bytes[0], bytes[1] = the
+ * algorithmic DRAM bytes per iteration (stencil: r, p read, p, Ap written;
+ * update: p, r, Ap read, r written, and x read and written once a group; 8 B
+ * each per unknown). */
 int pot3d_gpu_time_kernels(pot3d_gpu_solver *s, int reps, double ms[2], double bytes[2]);
 /* Average device milliseconds of the ILU(0) forward (ms[0]) and backward
  * (ms[1]) wavefront sweeps over `reps` applications (ifprec = 2 only), in

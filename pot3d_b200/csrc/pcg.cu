@@ -1725,8 +1725,10 @@ int Solver::cgsolve_padded(bool zero_guess, int ncgmax, double epscg, int *ierr,
   return POT3D_OK;
 }
 
-// Stencil and update kernels of the FP64 diagonal PCG timed one by one.
+// Stencil and update kernels of the FP64 diagonal PCG timed one by one, in the
+// form the solver iterates with (the grouped x update counts with the update).
 int Solver::time_kernels(int reps, double ms[2], double bytes[2]) {
+  reps = (reps + xg64 - 1) / xg64 * xg64;  // whole groups
   dim3 grid(g.nit, g.njt, g.nkc);
   dim3 gridu(g.nit, g.njt, g.nkc_u);
   SolveState s0{};
@@ -1756,6 +1758,12 @@ int Solver::time_kernels(int reps, double ms[2], double bytes[2]) {
   p_nxt = d_p2;
   for (int it = 0; it < reps; it++) {
     StencilArgs sa{};
+    if (xg64 > 1) {
+      p_cur = m_p64q[it % xg64];
+      p_nxt = m_p64q[(it + 1) % xg64];
+      sa.xslot1 = 1 + it % xg64;
+      ua.x = nullptr;
+    }
     sa.p_old = p_cur;
     sa.p_new = p_nxt;
     sa.r = d_r;
@@ -1775,6 +1783,7 @@ int Solver::time_kernels(int reps, double ms[2], double bytes[2]) {
     k_stencil<MODE_PCG><<<grid, NTHR, StageLayout<MODE_PCG>::smem, stream>>>(mp, g, m, sa);
     CK(cudaEventRecord(e[1], stream));
     k_update<UPD_ITER, false><<<gridu, NTHR, 0, stream>>>(g, m, ua);
+    if (xg64 > 1 && it % xg64 == xg64 - 1 && (stm = launch_x_group(m_p64q))) return stm;
     CK(cudaEventRecord(e[2], stream));
     CK(cudaEventSynchronize(e[2]));
     float a = 0.f, b = 0.f;
@@ -1794,7 +1803,7 @@ int Solver::time_kernels(int reps, double ms[2], double bytes[2]) {
   ms[0] = t0 / reps;
   ms[1] = t1 / reps;
   bytes[0] = 32.0 * (double)g.N;
-  bytes[1] = 48.0 * (double)g.N;
+  bytes[1] = (32.0 + 16.0 / xg64) * (double)g.N;
   return POT3D_OK;
 }
 

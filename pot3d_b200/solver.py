@@ -185,8 +185,8 @@ class Pot3dSolver:
         return float(ms[0]), float(ms[1])
 
     def time_kernels(self, reps: int = 20):
-        """Average ms per launch of the stencil and update kernels, and their
-        algorithmic DRAM bytes per launch."""
+        """Average ms per iteration of the stencil and update kernels, and their
+        algorithmic DRAM bytes per iteration."""
         ms = np.zeros(2)
         by = np.zeros(2)
         check(_lib.lib().pot3d_gpu_time_kernels(self._h, reps, dptr(ms), dptr(by)))

@@ -46,3 +46,9 @@ def test_reference_arm_needs_the_oracle_fixture_on_large_grids():
     out = _run("--impl", "reference", "--steps", "1", "--warmup", "0", "--workload", "pfss_127x181x361",
                "--ifprec", "2")
     assert out.returncode != 0 and "make_c2_oracle.py" in (out.stderr + out.stdout)
+
+
+def test_bytes_of_an_iteration():
+    import bench
+    assert bench.bytes_per_iteration("fp64", 1, 1) == 80.0 and bench.bytes_per_iteration("fp64", 1, 4) == 68.0
+    assert bench.bytes_per_iteration("fp32_refined", 2, 8) == 58.0 and bench.bytes_per_iteration("fp64", 2, 1) == 104.0

@@ -68,6 +68,16 @@ def test_refined_groups_follow_fp64(cuda, case, ifprec):
             assert np.linalg.norm(y - x) <= 64 * n * 2.0 ** -24 * np.linalg.norm(x), n
 
 
+def test_kernel_times_count_the_bytes_of_groups(cuda, case):
+    mesh, br0 = case
+    with Pot3dSolver(mesh, br0) as s:
+        ms, by = s.time_kernels(5)
+        assert np.all(ms > 0) and by[0] == 32.0 * s.N and by[1] == 36.0 * s.N
+        x, _ = _x(s, s.rhs(), 5)  # and leaves the handle as it was
+    with Pot3dSolver(mesh, br0) as s:
+        assert np.array_equal(x, _x(s, s.rhs(), 5)[0])
+
+
 def test_grids_within_l2_update_every_iteration(cuda):
     mesh = host.make_mesh(33, 41, 65)
     br0 = host.br0_from_map(mesh, *host.synthetic_br(4, 15, 4, mesh.nt, mesh.np))
