@@ -585,7 +585,9 @@ struct UpdateArgs {
 
 // R32: the residual (and, for UPD_ITER, p and q) are FP32 vectors; the
 // arithmetic is FP64 and the new residual is rounded once when stored.
-template <int KIND, bool ZIN, bool R32 = false>
+// X: UPD_ITER also updates x; without, x is left to k_update_x_group.
+// S: planes whose loads are issued ahead of the first plane's stores.
+template <int KIND, bool ZIN, bool R32, bool X, int S>
 __device__ __forceinline__ void update_body(const Geo &g, const DevMesh &m, const UpdateArgs &a, const int bx,
                                             const int by, const int bz) {
   __shared__ double red[NTHR / 32];
@@ -603,55 +605,83 @@ __device__ __forceinline__ void update_body(const Geo &g, const DevMesh &m, cons
   const bool v1 = v0 && e0 + 1 < g.nrm2;
   const bool south = v0 && jj == g.ntm2 - 1;
   double rz = 0.0, s1a = 0.0, s1b = 0.0;
-  if (v0) {
-#pragma unroll 4
-    for (int kk = k0; kk < k1; kk++) {
-      const long long id = g.idx(e0, jj, kk);
-      // q, p and z come from the kernels before: ordinary loads (see pdl_wait),
-      // q's ahead of x's store
-      double2 rv = R32 ? widen2(*reinterpret_cast<const float2 *>(a.r32 + id))
-                       : *reinterpret_cast<const double2 *>(a.r + id);
+  // r, q, p and z come from the kernels before: ordinary loads (see pdl_wait)
+  using V = typename std::conditional<R32, float2, double2>::type;
+  auto wide = [](V v) {
+    if constexpr (R32)
+      return widen2(v);
+    else
+      return v;
+  };
+  V *rv;
+  const V *qv, *pv;
+  if constexpr (R32) {
+    rv = reinterpret_cast<V *>(a.r32);
+    qv = reinterpret_cast<const V *>(a.q32);
+    pv = reinterpret_cast<const V *>(a.p32);
+  } else {
+    rv = reinterpret_cast<V *>(a.r);
+    qv = reinterpret_cast<const V *>(a.q);
+    pv = reinterpret_cast<const V *>(a.p);
+  }
+  double2 *const xv = reinterpret_cast<double2 *>(a.x);
+  const long long step = (long long)g.NRP * g.ntm2 / 2;
+  auto planes = [&](auto nc, int kk) {
+    constexpr int N = decltype(nc)::value;
+    const long long id0 = g.idx(e0, jj, kk) / 2;
+    V r0[N], q0[N], p0[N];
+    double2 x0[N];
+    float2 z0[N];
+#pragma unroll
+    for (int s = 0; s < N; s++) {
+      const long long id = id0 + s * step;
+      r0[s] = rv[id];
+      if (KIND == UPD_ITER) q0[s] = qv[id];
+      if (X) {
+        x0[s] = xv[id];
+        p0[s] = pv[id];
+      }
+      z0[s] = ZIN ? reinterpret_cast<const float2 *>(a.z32)[id] : __ldg(reinterpret_cast<const float2 *>(a.ai) + id);
+    }
+#pragma unroll
+    for (int s = 0; s < N; s++) {
+      const long long id = id0 + s * step;
+      if (X) {
+        const double2 p = wide(p0[s]);
+        xv[id] = make_double2(fma(alpha, p.x, x0[s].x), fma(alpha, p.y, x0[s].y));
+      }
+      double2 r = wide(r0[s]);
       if (KIND == UPD_ITER) {
-        const double2 qv = R32 ? widen2(*reinterpret_cast<const float2 *>(a.q32 + id))
-                               : *reinterpret_cast<const double2 *>(a.q + id);
-        if (a.x) {  // else applied in groups of iterations (k_update_x_group)
-          double2 xv = *reinterpret_cast<const double2 *>(a.x + id);
-          const double2 pv = R32 ? widen2(*reinterpret_cast<const float2 *>(a.p32 + id))
-                                 : *reinterpret_cast<const double2 *>(a.p + id);
-          xv.x = fma(alpha, pv.x, xv.x);
-          xv.y = fma(alpha, pv.y, xv.y);
-          *reinterpret_cast<double2 *>(a.x + id) = xv;
-        }
-        rv.x = fma(-alpha, qv.x, rv.x);
-        rv.y = fma(-alpha, qv.y, rv.y);
-        if (R32) {
-          const float2 r2 = make_float2((float)rv.x, (float)rv.y);
-          *reinterpret_cast<float2 *>(a.r32 + id) = r2;
-          rv = widen2(r2);  // r.z of the stored residual
+        const double2 q = wide(q0[s]);
+        r.x = fma(-alpha, q.x, r.x);
+        r.y = fma(-alpha, q.y, r.y);
+        if constexpr (R32) {
+          const float2 r2 = make_float2((float)r.x, (float)r.y);
+          rv[id] = r2;
+          r = widen2(r2);  // r.z of the stored residual
         } else {
-          *reinterpret_cast<double2 *>(a.r + id) = rv;
+          rv[id] = r;
         }
       }
-      if (!v1) rv.y = 0.0;
-      double zx, zy;
-      if (ZIN) {
-        const float2 zv = *reinterpret_cast<const float2 *>(a.z32 + id);
-        zx = zv.x;
-        zy = zv.y;
-      } else {
-        const float2 av = __ldg(reinterpret_cast<const float2 *>(a.ai + id));
-        zx = (double)av.x * rv.x;
-        zy = (double)av.y * rv.y;
-      }
+      if (!v1) r.y = 0.0;
+      const double zx = ZIN ? (double)z0[s].x : (double)z0[s].x * r.x;
+      double zy = ZIN ? (double)z0[s].y : (double)z0[s].y * r.y;
       if (!v1) zy = 0.0;
-      rz = fma(rv.x, zx, rz);
-      rz = fma(rv.y, zy, rz);
+      rz = fma(r.x, zx, rz);
+      rz = fma(r.y, zy, rz);
       if (south && KIND != UPD_BDOTB) {
-        const double wk = m.dph[kk + 2];
+        const double wk = m.dph[kk + s + 2];
         s1a += __dmul_rn(zx, wk) * m.pl_i;
         s1b += __dmul_rn(zy, wk) * m.pl_i;
       }
     }
+  };
+  if (v0) {
+    int kk = k0;
+    if (S > 1)
+      for (; kk + S <= k1; kk += S) planes(std::integral_constant<int, S>{}, kk);
+#pragma unroll (S > 1 ? 1 : 4)
+    for (; kk < k1; kk++) planes(std::integral_constant<int, 1>{}, kk);
   }
   if (south && KIND != UPD_BDOTB) {
     a.s1z_part[(long long)bz * g.NRP + e0] = s1a;
@@ -673,11 +703,21 @@ __device__ __forceinline__ void update_body(const Geo &g, const DevMesh &m, cons
   }
 }
 
-// Six blocks an SM (40 registers), four of the batched form: without the bound
-// the ordinary loads of four planes are hoisted into 54 registers.
-template <int KIND, bool ZIN, bool R32 = false>
-__global__ void __launch_bounds__(NTHR, 6) k_update(Geo g, DevMesh m, UpdateArgs a) {
-  update_body<KIND, ZIN, R32>(g, m, a, blockIdx.x, blockIdx.y, blockIdx.z);
+// Planes ahead (S) and blocks an SM.  Ordinary loads do not pass the stores of
+// the planes before, so a form says how many planes it loads first; with one
+// plane at a time and 40 registers, as with the read-only loads it had, a solve
+// took 6.04 s at 255x361x721 FP64, 455 ms at 121x181x361, 298 at 127x181x361
+// refined, 33.3 at 63x91x181.  Without x: FP64 four planes and three blocks
+// (5.87 s, 441 ms; 8 planes 5.99 and 449, 2 planes at six blocks 5.91 and 448),
+// refined two and six (286 ms; 4 at four 295, 4 at five 309).  With x, on grids
+// within L2: one plane, five blocks (32.0 ms; 2 planes 33.1).  Batches: two
+// planes, four blocks (six grids of 63 to 127 x 91 to 181 x 181 to 361: 1194 ms
+// FP64, 1042 refined; one plane 1193 and 1088).
+constexpr int upd_planes(int kind, bool r32, bool x) { return kind != UPD_ITER || x ? 1 : r32 ? 2 : 4; }
+constexpr int upd_blocks(int kind, bool r32, bool x) { return kind != UPD_ITER ? 6 : x ? 5 : r32 ? 6 : 3; }
+template <int KIND, bool ZIN, bool R32 = false, bool X = KIND == UPD_ITER>
+__global__ void __launch_bounds__(NTHR, upd_blocks(KIND, R32, X)) k_update(Geo g, DevMesh m, UpdateArgs a) {
+  update_body<KIND, ZIN, R32, X, upd_planes(KIND, R32, X)>(g, m, a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // ifprec=2 half of the update: x += alpha p ; r -= alpha q ; r32 = (float)r
@@ -1288,7 +1328,7 @@ int Solver::setup(const pot3d_mesh_t *mesh, const double *br0, const double *br1
   // pick the chunk count that minimises whole waves x planes per block,
   // counting each block's pipeline start-up as extra planes.
   {
-    int dev = 0, nsm = 148, occ_s = 2, occ_u = 8;
+    int dev = 0, nsm = 148, occ_s = 2;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     // occupancy of the stencil form this solver iterates with (the ILU(0)
@@ -1303,7 +1343,6 @@ int Solver::setup(const pot3d_mesh_t *mesh, const double *br0, const double *br1
                                                        StageLayout<MODE_PCG32>::smem));
     else
       CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_stencil<MODE_PCG>, NTHR, StageLayout<MODE_PCG>::smem));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, k_update<UPD_ITER, false>, NTHR, 0));
     const long long cols = (long long)g.nit * g.njt;
     auto pick = [&](int slots_per_sm, double startup, int max_tk, int *tk, int *nkc) {
       const double slots = (double)std::max(1, slots_per_sm) * nsm;
@@ -1322,7 +1361,7 @@ int Solver::setup(const pot3d_mesh_t *mesh, const double *br0, const double *br1
       }
     };
     pick(occ_s, 6.0, MAX_TK, &g.tk, &g.nkc);
-    pick(occ_u, 2.0, 1 << 30, &g.tk_u, &g.nkc_u);
+    pick(6, 2.0, 1 << 30, &g.tk_u, &g.nkc_u);  // six blocks for every form: the order of r.z is the same in all
   }
   CK(cudaEventCreate(&ev0));
   CK(cudaEventCreate(&ev1));
@@ -1558,12 +1597,10 @@ int Solver::launch_iteration(int u) {
   } else {
     if ((stm = tensor_map(d_r, true, &mp.m64[1]))) return stm;
     if ((stm = tensor_map(d_ai, false, &mp.m32[0]))) return stm;
-    if (xg64 > 1) {
-      sa.xslot1 = 1 + u % xg64;
-      ua.x = nullptr;
-    }
+    if (xg64 > 1) sa.xslot1 = 1 + u % xg64;
     CK(launch_pdl(k_stencil<MODE_PCG>, grid, dim3(NTHR), StageLayout<MODE_PCG>::smem, stream, mp, g, m, sa));
-    CK(launch_pdl(k_update<UPD_ITER, false, false>, gridu, dim3(NTHR), 0, stream, g, m, ua));
+    CK(launch_pdl(xg64 > 1 ? k_update<UPD_ITER, false, false, false> : k_update<UPD_ITER, false, false, true>, gridu,
+                  dim3(NTHR), 0, stream, g, m, ua));
     int st;
     if (xg64 > 1 && u % xg64 == xg64 - 1 && (st = launch_x_group(m_p64q))) return st;
   }
@@ -1762,7 +1799,6 @@ int Solver::time_kernels(int reps, double ms[2], double bytes[2]) {
       p_cur = m_p64q[it % xg64];
       p_nxt = m_p64q[(it + 1) % xg64];
       sa.xslot1 = 1 + it % xg64;
-      ua.x = nullptr;
     }
     sa.p_old = p_cur;
     sa.p_new = p_nxt;
@@ -1782,7 +1818,10 @@ int Solver::time_kernels(int reps, double ms[2], double bytes[2]) {
     CK(cudaEventRecord(e[0], stream));
     k_stencil<MODE_PCG><<<grid, NTHR, StageLayout<MODE_PCG>::smem, stream>>>(mp, g, m, sa);
     CK(cudaEventRecord(e[1], stream));
-    k_update<UPD_ITER, false><<<gridu, NTHR, 0, stream>>>(g, m, ua);
+    if (xg64 > 1)
+      k_update<UPD_ITER, false, false, false><<<gridu, NTHR, 0, stream>>>(g, m, ua);
+    else
+      k_update<UPD_ITER, false><<<gridu, NTHR, 0, stream>>>(g, m, ua);
     if (xg64 > 1 && it % xg64 == xg64 - 1 && (stm = launch_x_group(m_p64q))) return stm;
     CK(cudaEventRecord(e[2], stream));
     CK(cudaEventSynchronize(e[2]));
@@ -1904,9 +1943,9 @@ int Solver::launch_iteration32(int u) {
     k_south_ring_z<<<dim3((g.nrm2 + 127) / 128, g.nkc_u), 128, 0, stream>>>(g, m, (const float *)dilu_z32(this), d_s1z);
   } else {
     if ((stm = tensor_map(m_r32, false, &mp.m32[1])) || (stm = tensor_map(d_ai, false, &mp.m32[2]))) return stm;
-    if (xg > 1) ua.x = nullptr;
     CK(launch_pdl(k_stencil<MODE_PCG32>, grid, dim3(NTHR), StageLayout<MODE_PCG32>::smem, stream, mp, g, m, sa));
-    CK(launch_pdl(k_update<UPD_ITER, false, true>, gridu, dim3(NTHR), 0, stream, g, m, ua));
+    CK(launch_pdl(xg > 1 ? k_update<UPD_ITER, false, true, false> : k_update<UPD_ITER, false, true, true>, gridu,
+                  dim3(NTHR), 0, stream, g, m, ua));
     int st;
     if (xg > 1 && u % xg == xg - 1 && (st = launch_x_group(m_p32q))) return st;
   }
@@ -2211,7 +2250,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_update_batch(const BatchInst *__res
   const BatchInst &I = in[i];
   const Geo &g = I.g;
   const unsigned local = blockIdx.x - I.off_u;
-  update_body<KIND, ZIN, R32>(g, I.m, I.ua[par], local % g.nit, (local / g.nit) % g.njt, local / (g.nit * g.njt));
+  update_body<KIND, ZIN, R32, KIND == UPD_ITER, 2>(g, I.m, I.ua[par], local % g.nit, (local / g.nit) % g.njt, local / (g.nit * g.njt));
 }
 
 __global__ void __launch_bounds__(NTHR) k_update_r32_batch(const BatchInst *__restrict__ in, int n, int par) {

@@ -31,7 +31,7 @@ def _functions(src):
 def test_overlapped_kernels_read_only_setup_data_through_the_read_only_path():
     src = _source("pcg.cu")
     fn = _functions(src)
-    launched = set(re.findall(r"launch_pdl\((\w+)", src))
+    launched = {k for call in re.findall(r"launch_pdl\(([^;]*);", src) for k in re.findall(r"\bk_\w+\b(?!\")", call)}
     assert launched == {"k_stencil", "k_update", "k_update_x_group"}
     for k in launched:
         bodies = [fn[k]] + [fn[c] for c in re.findall(r"\b(\w+_body)\b", fn[k])]
