@@ -726,10 +726,11 @@ __global__ void __launch_bounds__(256) k_guess(const float *__restrict__ out, lo
 // output, and conversions issue at a tenth of the FP32 rate; STAGED converts a
 // row once into shared memory, a warp a row (182 -> 150 us for 125 -> 253
 // levels at 359 x 719 positions): where the outputs need at least the row's
-// conversions, for rows of up to 768 values, where eight fit 48 KB.
+// conversions, for rows of up to 768 values, where eight fit 48 KB.  The whole
+// row, its padding too, so that every index that is inside a row stays inside.
 template <bool STAGED>
 __global__ void __launch_bounds__(256) k_guess_resampled(const float *__restrict__ out, long long B, long long npos,
-                                                         int Rp, int Rs, const int *__restrict__ idx,
+                                                         int Rp, const int *__restrict__ idx,
                                                          const double *__restrict__ w, int R,
                                                          const double *__restrict__ sigma, double *__restrict__ x) {
   if (!STAGED) {
@@ -742,12 +743,12 @@ __global__ void __launch_bounds__(256) k_guess_resampled(const float *__restrict
   }
   extern __shared__ double row_s[];
   const int lane = threadIdx.x & 31;
-  double *row = row_s + (threadIdx.x >> 5) * Rs;
+  double *row = row_s + (threadIdx.x >> 5) * Rp;
   for (long long bp = blockIdx.x * 8LL + (threadIdx.x >> 5); bp < B * npos; bp += gridDim.x * 8LL) {
     const double sg = sigma[bp / npos];
     const float *o = out + bp * Rp;
 #pragma unroll 4
-    for (int i = lane; i < Rs; i += 32) row[i] = (double)o[i];
+    for (int i = lane; i < Rp; i += 32) row[i] = (double)o[i];
     __syncwarp();
 #pragma unroll 4
     for (int i = lane; i < R; i += 32) {
@@ -767,12 +768,12 @@ extern "C" int pot3d_fno_guess_resampled(const float *out, long long B, long lon
     pot3d_set_error("pot3d_fno_guess_resampled: bad sizes");
     return POT3D_ERR_ARG;
   }
-  const size_t smem = 8 * sizeof(double) * (size_t)Rs;  // a row for each of the eight warps
-  if (smem <= 48 * 1024 && 2LL * R >= Rs && !by_elements(B * npos, R))
-    k_guess_resampled<true><<<grid_for(B * npos * 32), 256, smem, (cudaStream_t)stream>>>(out, B, npos, Rp, Rs, idx, w, R,
+  const size_t smem = 8 * sizeof(double) * (size_t)Rp;  // a row for each of the eight warps
+  if (smem <= 48 * 1024 && 2LL * R >= Rp && !by_elements(B * npos, R))
+    k_guess_resampled<true><<<grid_for(B * npos * 32), 256, smem, (cudaStream_t)stream>>>(out, B, npos, Rp, idx, w, R,
                                                                                           sigma, x);
   else
-    k_guess_resampled<false><<<rows_grid(B * npos, R), 256, 0, (cudaStream_t)stream>>>(out, B, npos, Rp, Rs, idx, w, R,
+    k_guess_resampled<false><<<rows_grid(B * npos, R), 256, 0, (cudaStream_t)stream>>>(out, B, npos, Rp, idx, w, R,
                                                                                       sigma, x);
   return pot3d_cuda_status(cudaGetLastError(), "pot3d_fno_guess_resampled");
 }

@@ -214,14 +214,15 @@ def test_gelu_and_guess_of_any_width(cuda, rows, c, ldo):
 
 
 @pytest.mark.parametrize("b,npos,rs,r", [(1, 1, 2, 1), (2, 1201, 125, 253), (1, 2500, 768, 800), (1, 9, 769, 31),
-                                         (2, 1500, 125, 31), (1, 2100, 125, 62), (3, 800, 70, 33)])
+                                         (2, 1500, 125, 31), (1, 2100, 125, 62), (3, 800, 70, 33), (1, 2500, 70, 70)])
 def test_guess_resampled(cuda, b, npos, rs, r):
     import torch
     from pot3d_b200 import _lib
     from pot3d_b200.fno import _L
     rp = (rs + 63) // 64 * 64
     out = _t((b, npos, rp), cuda, 12)
-    idx = torch.randint(0, rs - 1, (r,), device=cuda, dtype=torch.int32, generator=torch.Generator(cuda).manual_seed(13))
+    hi = rp - 1 if (rs, r) == (70, 70) else rs - 1  # once every index inside a row, padding included
+    idx = torch.randint(0, hi, (r,), device=cuda, dtype=torch.int32, generator=torch.Generator(cuda).manual_seed(13))
     w, sigma = 1.2 * _t((r,), cuda, 14, torch.float64), _t((b,), cuda, 15, torch.float64)
     x = torch.empty((b, npos, r), device=cuda, dtype=torch.float64)
     _lib.check(_L().pot3d_fno_guess_resampled(*[C.c_void_p(out.data_ptr()), b, npos, rp, rs], C.c_void_p(idx.data_ptr()),
