@@ -159,8 +159,9 @@ __device__ __forceinline__ double apply_fac(const PtFac &f, double dpim, double 
 // A thread marches along k with its own column's three planes in registers
 // and reads only the neighbours in e and j from shared memory, two columns per
 // access.  Measured against every neighbour read from the ring: PCGZ32 53.8 ->
-// 49.9 us at 127x181x361; whole solves, 127x181x361 FP32-refined diagonal 336
-// -> 302 ms and 121x181x361 FP64 diagonal 506 -> 455 ms.
+// 49.9 us at 127x181x361 (344 -> 315 at 255x361x721); whole solves, 127x181x361
+// FP32-refined diagonal 336 -> 302 ms and 121x181x361 FP64 diagonal 506 -> 455
+// to 475 ms.
 // ============================================================================
 enum { MODE_AX = 0, MODE_PCG = 1, MODE_PCGZ = 2, MODE_PCG32 = 3, MODE_PCGZ32 = 4 };
 
